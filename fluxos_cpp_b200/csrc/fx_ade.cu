@@ -1,4 +1,5 @@
-// FP64 advection-dispersion (ADE) step of FLUXOS-OVERLAND for sm_100a.
+// Advection-dispersion (ADE) step of FLUXOS-OVERLAND for sm_100a, the form for
+// launches with many units in flight (fx_ade_chain.cu has the one for few).
 //
 // ADEsolver_calc.cpp:27-291 re-scales every concentration to the new depth
 // (:47-73) and then sweeps the grid once in Gauss-Seidel order (:93-290):
@@ -41,6 +42,7 @@
 #include <vector>
 
 #include "fx_common.cuh"
+#include "fx_internal.h"
 
 namespace fxade {
 
@@ -62,10 +64,8 @@ constexpr long long HOLD_SPIN_LIMIT = 1LL << 12;  // the same with fx_dev.ade_ho
 template <class T>
 struct Ring;
 // The FP64 ring: the concentration group, the cell's six per-step values
-// {h0, h, hp, fe_1, fn_1, flag bits} and the melt multiplier. A context's
-// record (fx_dev::rec64) lands in r as three 16-byte copies; the separate
-// arrays of fx_adesolver_noalloc land in the same places one by one (the
-// flag as the 4-byte word holding it, in r[5]'s low half).
+// {h0, h, hp, fe_1, fn_1, flag bits}, whose record (fx_dev::rec64) lands in r
+// as three 16-byte copies, and the melt multiplier.
 template <>
 struct Ring<double> {
   static constexpr int CV = 2;
@@ -102,10 +102,6 @@ template <class T>
 struct Fields;
 template <>
 struct Fields<double> {
-  static __device__ __forceinline__ const double* h(const fx_dev& d) { return d.h; }
-  static __device__ __forceinline__ const double* h0(const fx_dev& d) { return d.h0; }
-  static __device__ __forceinline__ const double* fe1(const fx_dev& d) { return d.fe1; }
-  static __device__ __forceinline__ const double* fn1(const fx_dev& d) { return d.fn1; }
   static __device__ __forceinline__ const double* mm(const fx_dev& d) { return d.melt_mult; }
   static __device__ __forceinline__ double* conc(const fx_dev& d) { return d.conc; }
   static __device__ __forceinline__ double* soil(const fx_dev& d) { return d.soil; }
@@ -196,18 +192,8 @@ __device__ __forceinline__ void prefetch(const fx_dev& d, const StepIn& S, const
   } else {
     double* re = &R.r[slot][lane][0];
     const unsigned e = (unsigned)__cvta_generic_to_shared(re);
-    if (d.rec64) {  // a context: the cell's record, 48 bytes
-      const double* rec = fx_rec64(d, o);
-      for (int q = 0; q < 3; ++q) cp_async_sz(e + 16 * q, rec + 2 * q, inr ? 16 : 0, 16);
-    } else {  // fx_adesolver_noalloc: the caller's arrays (no melt, no slots)
-      const int nb = inr ? 8 : 0;
-      cp_async_sz(e + 8 * FX_R64_H0, F::h0(d) + o, nb, 8);
-      cp_async_sz(e + 8 * FX_R64_H, F::h(d) + o, nb, 8);
-      cp_async_sz(e + 8 * FX_R64_FE1, F::fe1(d) + o, nb, 8);
-      cp_async_sz(e + 8 * FX_R64_FN1, F::fn1(d) + o, nb, 8);
-      // the 4-byte word holding the flag byte (planes are multiples of 32 bytes)
-      cp_async_sz(e + 8 * FX_R64_FL, d.flags + (o & ~3LL), inr ? 4 : 0, 4);
-    }
+    const double* rec = fx_rec64(d, o);  // the cell's record, 48 bytes
+    for (int q = 0; q < 3; ++q) cp_async_sz(e + 16 * q, rec + 2 * q, inr ? 16 : 0, 16);
     const bool mm_ok = S.dilute && F::mm(d) != nullptr;
     cp_async_sz((unsigned)__cvta_generic_to_shared(&R.mm[slot][lane]),
                 mm_ok ? (const void*)(F::mm(d) + gi) : (const void*)d.flags, mm_ok && inr ? 8 : 0, 8);
@@ -234,9 +220,7 @@ __device__ __forceinline__ Rec<T> make_rec_br(const fx_dev& d, const StepIn& S, 
   r.h = v[FX_R64_H];
   if (ix >= 1 && ix <= d.nr && iy >= 1 && iy <= d.nc) {
     const long long gi = fx_ix(d, ix, iy);
-    // a record holds the flag byte itself, a separate flags array the word holding it
-    const unsigned word = (unsigned)__double_as_longlong(v[FX_R64_FL]);
-    const unsigned fl = (d.rec64 ? word : word >> (8 * (unsigned)(gi & 3))) & 0xffu;
+    const unsigned fl = (unsigned)__double_as_longlong(v[FX_R64_FL]) & 0xffu;
     r.ld = fl & FX_F_LDRY;
     const int ldp = (fl & FX_F_LDRY_PREV) ? 1 : 0;
     T c = R.c[slot][lane][gi & (Ring<T>::CV - 1)];
@@ -918,16 +902,43 @@ __global__ void __launch_bounds__(WARPS * 32, AdeBlocks<T>::value) k_ade_batch(c
 }  // namespace fxade
 
 int fx_ade_rows_per_strip() { return fxade::ROWS; }
-int fx_ade_threads_per_block() { return fxade::WARPS * 32; }
 static size_t ade_smem(bool prec32) {
   return (prec32 ? sizeof(fxade::Ring<float>) : sizeof(fxade::Ring<double>)) * fxade::WARPS;
 }
 
-void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, int nblocks, bool prec32, cudaStream_t s) {
+// Units of a domain's launch that are at work at the same time when only
+// their dependencies hold them back: their warp steps over the warp steps of
+// the launch (a strip follows its west strip by about 37 of them, a step the
+// step before by about 48).
+double fx_ade_active(int nr, int nc, int nchem, int steps) {
+  const double strips = (nr + fxade::ROWS - 1) / fxade::ROWS, tw = nc + fxade::ROWS - 1;
+  return steps * nchem * strips * tw / (37.0 * strips + 48.0 * steps + nc);
+}
+// Which kernel. The chain kernel (a block per unit) takes a unit through its
+// warp steps 3 to 5 times faster but holds 2 (FP64) or 3 (FP32) units per SM
+// against 12, so it wins until the units at work are about its own: 1.8x (FP32)
+// and 2.5x (FP64) at 0.65 units per SM (400^2, 63 steps), 1.5x and 1.7x at 1.6
+// (2048^2, 8 steps), 1.13x and 1.04x at 3.2 (4096^2, 8 steps), 0.97x and
+// 0.92x at 3.5 (2048^2, 20 steps), 0.93x and 0.6x at 6 (1024^2, three solutes).
+bool fx_ade_use_chain(const fx_ade_caps& caps, double active) { return active <= 3.25 * caps.sms; }
+
+void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const fx_ade_caps& caps, bool chain, bool prec32,
+                   cudaStream_t s) {
+  if (chain) {
+    fx_chain_launch(devs, units, nunits, caps.chain, prec32, s);
+    return;
+  }
+  const int nblocks = std::max(1, std::min((nunits + fxade::WARPS - 1) / fxade::WARPS, caps.sweep));
   if (prec32) fxade::k_ade_batch<float><<<nblocks, fxade::WARPS * 32, ade_smem(true), s>>>(devs, units, nunits);
   else fxade::k_ade_batch<double><<<nblocks, fxade::WARPS * 32, ade_smem(false), s>>>(devs, units, nunits);
 }
-void fx_launch_ade_one(const fx_dev& d, int nunits, int nblocks, cudaStream_t s) {
+void fx_launch_ade_one(const fx_dev& d, int steps, const fx_ade_caps& caps, cudaStream_t s) {
+  const int nunits = steps * d.nchem * ((d.nr + fxade::ROWS - 1) / fxade::ROWS);
+  if (fx_ade_use_chain(caps, fx_ade_active(d.nr, d.nc, d.nchem, steps))) {
+    fx_chain_launch_one(d, nunits, caps.chain, s);
+    return;
+  }
+  const int nblocks = std::max(1, std::min((nunits + fxade::WARPS - 1) / fxade::WARPS, caps.sweep));
   if (d.prec32) fxade::k_ade_one<float><<<nblocks, fxade::WARPS * 32, ade_smem(true), s>>>(d, nunits);
   else fxade::k_ade_one<double><<<nblocks, fxade::WARPS * 32, ade_smem(false), s>>>(d, nunits);
 }
@@ -977,7 +988,7 @@ static int max_blocks_of(K kernel, size_t smem, int nsm, int* out) {
 // Resident blocks of the sweep kernels of one precision on this device (the
 // smaller of the one-domain and batch forms), after raising their dynamic
 // shared memory limit.
-int fx_ade_max_blocks_for(bool prec32, int* out) {
+int fx_ade_caps_for(bool prec32, fx_ade_caps* out) {
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -1;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
@@ -991,22 +1002,7 @@ int fx_ade_max_blocks_for(bool prec32, int* out) {
         max_blocks_of(fxade::k_ade_batch<double>, ade_smem(false), nsm, &b))
       return -1;
   }
-  *out = std::min(a, b);
-  return 0;
-}
-
-// Resident blocks of the sweep kernels on this device (the smallest of the
-// four variants), after raising their dynamic shared memory limit.
-int fx_ade_max_blocks(int* out) {
-  int dev = 0, nsm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-  int a = 0, b = 0, c = 0, e = 0;
-  if (max_blocks_of(fxade::k_ade_one<double>, ade_smem(false), nsm, &a) ||
-      max_blocks_of(fxade::k_ade_one<float>, ade_smem(true), nsm, &b) ||
-      max_blocks_of(fxade::k_ade_batch<double>, ade_smem(false), nsm, &c) ||
-      max_blocks_of(fxade::k_ade_batch<float>, ade_smem(true), nsm, &e))
-    return -1;
-  *out = std::min(std::min(a, b), std::min(c, e));
-  return 0;
+  out->sms = nsm;
+  out->sweep = std::min(a, b);
+  return out->sweep > 0 ? fx_chain_blocks(prec32, &out->chain) : -1;
 }

@@ -32,7 +32,9 @@ struct fx_batch {
   fx_unit* d_units = nullptr;
   fx_tmaps* d_tmaps = nullptr;  // one set of tensor maps per member (batch tile shape)
   size_t cap_devs = 0, cap_tiles = 0, cap_units = 0, cap_tmaps = 0;
-  int ntiles = 0, nunits = 0, K = 1, ade_blocks = 1;
+  int ntiles = 0, nunits = 0, K = 1;
+  fx_ade_caps ade_caps;
+  bool ade_chain = false;  // which ADE kernel the graph holds
   bool use_tma = true;   // option "tma": the TMA-staged batch kernel where the members allow it
   bool hydro_tma = false;  // the current graph uses it
   int tma_blocks = 0;
@@ -134,14 +136,14 @@ static int rebuild(fx_batch* b) {
   FXB_CK(b, cudaStreamSynchronize(b->stream));
   b->ntiles = (int)tiles.size();
   b->nunits = (int)units.size();
-  int maxb = 0;
-  if (fx_ade_max_blocks_for(n > 0 && b->doms[0]->d.prec32 != 0, &maxb) != 0 || maxb < 1) {
+  if (fx_ade_caps_for(n > 0 && b->doms[0]->d.prec32 != 0, &b->ade_caps) != 0) {
     int r = fx_fail(nullptr, FX_ERR_CUDA, "occupancy query for the ADE sweep failed");
     b->err = fx_last_error(nullptr);
     return r;
   }
-  const int per_block = fx_ade_threads_per_block() / 32;
-  b->ade_blocks = std::max(1, std::min((b->nunits + per_block - 1) / per_block, maxb));
+  double active = 0.0;
+  for (fx_ctx* c : b->doms) active += c->p.ade ? fx_ade_active(c->g.nrows, c->g.ncols, c->g.nchem, b->K) : 0.0;
+  b->ade_chain = fx_ade_use_chain(b->ade_caps, active);
   if (b->graph) {
     cudaGraphExecDestroy(b->graph);
     b->graph = nullptr;
@@ -159,7 +161,7 @@ static int rebuild(fx_batch* b) {
       else
         fx_launch_hydro(b->d_devs, b->d_tiles, b->ntiles, prec32, b->tile_rows, b->stream);
     }
-    fx_launch_ade(b->d_devs, b->d_units, b->nunits, b->ade_blocks, prec32, b->stream);
+    fx_launch_ade(b->d_devs, b->d_units, b->nunits, b->ade_caps, b->ade_chain, prec32, b->stream);
     FXB_CK(b, cudaStreamEndCapture(b->stream, &g));
     cudaError_t e = cudaGraphInstantiate(&b->graph, g, 0);
     cudaGraphDestroy(g);

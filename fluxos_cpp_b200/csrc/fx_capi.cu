@@ -370,23 +370,15 @@ int fx_create(const fx_grid* g, const fx_params* p, fx_ctx** out) {
   if ((rc = dev_alloc(c, (void**)&d.ade_prog,
                       sizeof(unsigned long long) * (size_t)d.nslot * g->nchem * c->ade_strips)) != FX_OK)
     goto fail;
-  {
-    int maxb = 0;
-    if (fx_ade_max_blocks_for(d.prec32 != 0, &maxb) != 0 || maxb < 1) {
-      rc = fx_fail(c, FX_ERR_CUDA, "occupancy query for the ADE sweep failed");
-      goto fail;
-    }
-    const int units = c->batch_steps * g->nchem * c->ade_strips;
-    const int per_block = fx_ade_threads_per_block() / 32;
-    int want = (units + per_block - 1) / per_block;
-    c->ade_blocks = want < maxb ? want : maxb;
+  if (fx_ade_caps_for(d.prec32 != 0, &c->ade_caps) != 0) {
+    rc = fx_fail(c, FX_ERR_CUDA, "occupancy query for the ADE sweep failed");
+    goto fail;
   }
   {
     // this domain's tile table (domain 0 of a batch of one), sized for the
     // smallest tiles (most entries)
     std::vector<fx_tile> tiles;
     fx_tiles_of(0, g->nrows, g->ncols, 4, tiles);
-    c->nunits = c->batch_steps * g->nchem * c->ade_strips;
     if ((rc = dev_alloc(c, (void**)&c->d_tiles, sizeof(fx_tile) * tiles.size())) != FX_OK) goto fail;
     if ((rc = dev_alloc(c, (void**)&c->d_dev, sizeof(fx_dev))) != FX_OK) goto fail;
     if ((rc = set_tile_rows(c, 8)) != FX_OK) goto fail;
@@ -900,7 +892,7 @@ static void launch_batch(fx_ctx* c, int m) {
     fx_launch_finalize(c->d_dev, 1, c->stream);
     launch_hydro(c);
   }
-  fx_launch_ade_one(c->d, c->nunits, c->ade_blocks, c->stream);
+  fx_launch_ade_one(c->d, m, c->ade_caps, c->stream);
 }
 
 static int ensure_graph(fx_ctx* c) {
@@ -1062,7 +1054,7 @@ int fx_time_steps(fx_ctx* c, int n, double* ms_total, double* ms_hydro, double* 
     }
     if (erc) break;
     a = b;
-    fx_launch_ade_one(c->d, c->nunits, c->ade_blocks, c->stream);
+    fx_launch_ade_one(c->d, m, c->ade_caps, c->stream);
     if ((erc = record(&b))) break;
     ade.push_back({a, b});
   }

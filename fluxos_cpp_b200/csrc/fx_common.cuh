@@ -79,6 +79,8 @@ struct fx_ctl {
   double budget_out;
   double inflowi;     // point-inflow depth of the current step
   double iconc;       // and its concentration
+  int ade_next;       // next unit of the ADE launch (fx_ade.cu); 0 when a batch opens
+  int pad2_;
   fx_steprec rec[FX_MAX_SLOTS];  // per-slot record of the last steps
 };
 

@@ -1988,7 +1988,9 @@ __global__ void k_finalize(const fx_dev* __restrict__ devs, int ndom) {
 // Opens a batch of steps whose ADE sweeps run together (fx_ade.cu).
 __global__ void k_batch_begin(const fx_dev* __restrict__ devs, int ndom) {
   const int dom = blockIdx.x * blockDim.x + threadIdx.x;
-  if (dom < ndom) devs[dom].ctl->batch = devs[dom].ctl->batch + 1;
+  if (dom >= ndom) return;
+  devs[dom].ctl->batch = devs[dom].ctl->batch + 1;
+  devs[dom].ctl->ade_next = 0;
 }
 
 // Sets the bed flags that never change (NODATA bed) in every slot plane.

@@ -9,6 +9,13 @@
 #include "fluxos_gpu.h"
 #include "fx_common.cuh"
 
+// Resident blocks of the two ADE kernels on a device: the sweep of one warp
+// per unit (fx_ade.cu) and the one of a block per unit (fx_ade_chain.cu).
+struct fx_ade_caps {
+  int sweep = 0, chain = 0;
+  int sms = 0;  // SMs of the device
+};
+
 struct fx_ctx {
   fx_grid g{};
   fx_params p{};
@@ -20,11 +27,11 @@ struct fx_ctx {
   std::vector<void*> allocs;
   long long bytes = 0;
   int ade_strips = 0;
-  int ade_blocks = 0;
+  fx_ade_caps ade_caps;
   int batch_steps = 1;         // steps per batch (ADE sweeps in flight)
   fx_dev* d_dev = nullptr;     // device copy of d (a batch of one domain)
   fx_tile* d_tiles = nullptr;  // this domain's hydrodynamic tiles
-  int ntiles = 0, nunits = 0;  // hydrodynamic tiles; ADE units of a full batch
+  int ntiles = 0;              // hydrodynamic tiles
   bool dev_dirty = true;       // d changed since it was copied to d_dev
   long long dev_version = 0;   // counts changes of d (batches compare it)
   bool prepared = false;
@@ -78,8 +85,13 @@ int fx_hydro_batch_tma_blocks(bool prec32, int tile_rows, int* out);
 int fx_build_tmaps_for(fx_ctx* c, int tile_rows, fx_tmaps* out);
 bool fx_tma_fits(const fx_ctx* c, int tile_rows);
 void fx_launch_courant_scan(const fx_dev* devs, const fx_tile* tiles, int ntiles, int tile_rows, cudaStream_t s);
-void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, int nblocks, bool prec32, cudaStream_t s);
-void fx_launch_ade_one(const fx_dev& d, int nunits, int nblocks, cudaStream_t s);
+// chain: which of the two kernels (fx_ade_use_chain of the sum of the domains'
+// fx_ade_active). fx_launch_ade_one picks its own for the given steps.
+double fx_ade_active(int nr, int nc, int nchem, int steps);
+bool fx_ade_use_chain(const fx_ade_caps& caps, double active);
+void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const fx_ade_caps& caps, bool chain, bool prec32,
+                   cudaStream_t s);
+void fx_launch_ade_one(const fx_dev& d, int steps, const fx_ade_caps& caps, cudaStream_t s);
 void fx_launch_eta_from_z(const fx_dev& d, const double* z, cudaStream_t s);
 void fx_launch_mass(const fx_dev& d, double* out, cudaStream_t s);
 void fx_tiles_of(int dom, int nr, int nc, int tile_rows, std::vector<fx_tile>& out);
@@ -95,6 +107,8 @@ void fx_launch_results_write(const fx_dev& d, double h_min_print, const long lon
 bool fx_tile_rows_ok(int tile_rows);
 void fx_units_of(int dom, int nr, int nchem, int steps, std::vector<fx_unit>& out);
 int fx_ade_rows_per_strip();
-int fx_ade_threads_per_block();
-int fx_ade_max_blocks(int* out);
-int fx_ade_max_blocks_for(bool prec32, int* out);
+int fx_ade_caps_for(bool prec32, fx_ade_caps* out);
+// The ADE kernel with a block per unit (fx_ade_chain.cu).
+void fx_chain_launch(const fx_dev* devs, const fx_unit* units, int nunits, int max_blocks, bool prec32, cudaStream_t s);
+void fx_chain_launch_one(const fx_dev& d, int nunits, int max_blocks, cudaStream_t s);
+int fx_chain_blocks(bool prec32, int* out);

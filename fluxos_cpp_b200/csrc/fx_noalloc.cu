@@ -44,12 +44,8 @@
 
 #include "fluxos_gpu.h"
 #include "fx_common.cuh"
+#include "fx_internal.h"
 
-void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, int nblocks, bool prec32, cudaStream_t s);
-int fx_ade_rows_per_strip();
-int fx_ade_threads_per_block();
-int fx_ade_max_blocks(int* out);
-int fx_fail(fx_ctx* ctx, int code, const char* fmt, ...);
 
 #define FX_NOALLOC_SCRATCH_BYTES (8u << 20)
 
@@ -65,7 +61,7 @@ struct DeviceSetup {
   bool ready = false;
   unsigned long long ctx_id = 0;     // the CUDA context the set-up belongs to
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch
-  int max_blocks = 0;
+  int chain_blocks = 0;
 };
 DeviceSetup g_setup[kMaxDevices];
 std::mutex g_setup_mutex;
@@ -176,11 +172,11 @@ extern "C" int fx_adesolver_noalloc(double* conc, const double* h, const double*
       if (e != cudaSuccess || !p)
         return fx_fail(nullptr, FX_ERR_CUDA, "cudaGetSymbolAddress(g_noalloc_scratch) failed: %s",
                        cudaGetErrorString(e));
-      int mb = 0;
-      if (fx_ade_max_blocks(&mb) != 0 || mb < 1)
+      int blocks = 0;
+      if (fx_chain_blocks(false, &blocks) != 0)
         return fx_fail(nullptr, FX_ERR_CUDA, "occupancy query for the ADE sweep failed");
       g.scratch = (unsigned char*)p;
-      g.max_blocks = mb;
+      g.chain_blocks = blocks;
       g.ctx_id = current_context_id();  // the look-up made the device's context current
       g.ready = true;
     }
@@ -215,10 +211,7 @@ extern "C" int fx_adesolver_noalloc(double* conc, const double* h, const double*
   k_noalloc_setup<<<1, 128, 0, st>>>(d, d_dev, d_units, nstrips, dtfl);
   e = cudaMemsetAsync(d.ade_prog, 0, prog_bytes, st);
   if (e != cudaSuccess) return fx_fail(nullptr, FX_ERR_CUDA, "cudaMemsetAsync failed: %s", cudaGetErrorString(e));
-  const int per_block = fx_ade_threads_per_block() / 32;
-  int nblocks = (nstrips + per_block - 1) / per_block;
-  if (nblocks > s.max_blocks) nblocks = s.max_blocks;
-  fx_launch_ade(d_dev, d_units, nstrips, nblocks, false, st);
+  fx_chain_launch(d_dev, d_units, nstrips, s.chain_blocks, false, st);
   e = cudaGetLastError();
   if (e != cudaSuccess) return fx_fail(nullptr, FX_ERR_CUDA, "ADE sweep launch failed: %s", cudaGetErrorString(e));
   int err = 0;
