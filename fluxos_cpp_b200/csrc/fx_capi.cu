@@ -309,6 +309,7 @@ int fx_create(const fx_grid* g, const fx_params* p, fx_ctx** out) {
   d.nueml = (double)nuem;
   d.cvdefl = (double)cvdef;
   d.cfl_dxy = (double)(cfl * (float)g->dxy);
+  fx_set_f32(d);
   d.volrat_mode = p->volrat_mode;
   d.ade = p->ade;
   d.wintra = (p->wintra && p->ade) ? 1 : 0;  // main.cpp:209-213

@@ -84,6 +84,15 @@ struct fx_ctl {
   fx_steprec rec[FX_MAX_SLOTS];  // per-slot record of the last steps
 };
 
+// Constants of the FP32 arithmetic, rounded once on the host: a conversion
+// of an FP64 constant in a kernel takes the special-function unit (an eighth
+// of the issue rate) for every use that the registers do not keep.
+struct fx_f32 {
+  float hdry;              // dry threshold
+  float hdry_lo, hdry_hi;  // outside of these an FP32 depth decides the threshold tests (fx_hydro.cu)
+  float ks, gaccl, nueml, dxy, inv_dxy, area;
+};
+
 // Everything a kernel needs, passed by value.
 struct fx_dev {
   int nr, nc, ld, nchem;
@@ -98,6 +107,7 @@ struct fx_dev {
   double nueml;       // (double)(float)1.793e-6 (main.cpp:135)
   double cvdefl;      // (double)(float)0.07 (main.cpp:134)
   double cfl_dxy;     // (double)((float)cfl * (float)dxy) (main.cpp:316)
+  fx_f32 f;           // the same for the FP32 state
   int dxy_pow2;       // 1 when dxy is a power of two (then x/dxy == x*inv_dxy exactly)
   double inv_dxy;     // 1/dxy, exact when dxy_pow2
   double inv_area;    // 1/arbase, exact when dxy_pow2
@@ -192,16 +202,6 @@ struct fx_unit {
   int dom, jj, k, s;
 };
 
-// x / dxy and x / dxy^2. When dxy is a power of two the quotient is an
-// exact scaling, so multiplying by the exact reciprocal gives the same bits as
-// the division and saves a multi-instruction FP64 divide.
-__host__ __device__ inline double fx_div_dxy(const fx_dev& d, double x) {
-  return d.dxy_pow2 ? x * d.inv_dxy : x / d.dxy;
-}
-__host__ __device__ inline double fx_div_area(const fx_dev& d, double x) {
-  return d.dxy_pow2 ? x * d.inv_area : x / d.arbase;
-}
-
 inline void fx_set_cell_size(fx_dev& d, int dxy) {
   d.dxy_u = (unsigned)dxy;
   d.dxy = (double)dxy;
@@ -209,6 +209,19 @@ inline void fx_set_cell_size(fx_dev& d, int dxy) {
   d.dxy_pow2 = dxy > 0 && (dxy & (dxy - 1)) == 0 && dxy <= (1 << 20);
   d.inv_dxy = 1.0 / d.dxy;
   d.inv_area = 1.0 / d.arbase;
+}
+
+inline void fx_set_f32(fx_dev& d) {
+  d.f.hdry = (float)d.hdry;
+  const double band = (d.hdry < 0 ? -d.hdry : d.hdry) * 0x1p-19;
+  d.f.hdry_lo = (float)(d.hdry - band);
+  d.f.hdry_hi = (float)(d.hdry + band);
+  d.f.ks = (float)d.ks;
+  d.f.gaccl = (float)d.gaccl;
+  d.f.nueml = (float)d.nueml;
+  d.f.dxy = (float)d.dxy;
+  d.f.inv_dxy = (float)d.inv_dxy;
+  d.f.area = (float)d.arbase;
 }
 
 __host__ __device__ inline long long fx_ix(const fx_dev& d, int irow, int icol) {

@@ -63,8 +63,6 @@ struct HydroSmem {
   double u[VEL ? NSTEN : 1], v[VEL ? NSTEN : 1];
   double f[6][NFLUX];
   unsigned char cls[NSTEN];
-  short wet_list[NFLUX], dry_list[NFLUX], stale_list[NFLUX];
-  int nwet, ndry, nstale;
   double red_dt[NW], red_h[NW];
 };
 
@@ -85,6 +83,67 @@ __device__ __forceinline__ double fx_pow15(double h) {
   return p + (pe + h * slo);
 }
 
+// Quotients over a shared denominator, the bits of a / b: y = 1 / b, correctly
+// rounded, then two Newton corrections of a * y. The first leaves a faithful
+// quotient, so by Markstein's theorem (IBM J. Res. Dev. 34, 1990; Muller et al.,
+// Handbook of Floating-Point Arithmetic, ch. 4) the second rounds correctly; its
+// residual is exact for |a| >= 2^-700 and b, a below 2^200, 2^700. Anything else
+// divides, except 0, whose quotient is a * y (an FP64 division of 0 takes 436
+// cycles against 146 of an ordinary one, measured, and dry and resting cells
+// divide 0 all the time). The division stays out of line: a dozen copies of it
+// in the kernel cost more in instruction fetches than the quotients save
+// (2048 x 2048 cells 0.82 ms a step with them inline, 0.70 ms without, 0.80 ms
+// with plain divisions).
+__device__ __noinline__ double plain_div(double a, double b) { return a / b; }
+struct Over {
+  double b, y;
+  bool ok;
+  Over() = default;
+  __device__ __forceinline__ explicit Over(double b_) : b(b_), y(1.0 / b_) {
+    ok = (b > 6.223015277861142e-61) & (b < 1.6069380442589903e60);  // 2^-200, 2^200
+  }
+  __device__ __forceinline__ double of(double a) const {
+    const double q0 = a * y;
+    const double q1 = fma(fma(-b, q0, a), y, q0);
+    double q = fma(fma(-b, q1, a), y, q1);
+    const unsigned e = (unsigned)(__double2hiint(a) & 0x7ff00000) - ((1023u - 700u) << 20);
+    const bool zero = a == 0.0;
+    q = zero ? q0 : q;
+    if (!ok | ((e >= (1400u << 20)) & !zero)) q = plain_div(a, b);
+    return q;
+  }
+};
+// The same over a constant between 2^-200 and 2^200.
+__device__ __forceinline__ double over(double a, double b, double y) {
+  const double q0 = a * y;
+  const double q1 = fma(fma(-b, q0, a), y, q0);
+  double q = fma(fma(-b, q1, a), y, q1);
+  const unsigned e = (unsigned)(__double2hiint(a) & 0x7ff00000) - ((1023u - 700u) << 20);
+  const bool zero = a == 0.0;
+  q = zero ? q0 : q;
+  if ((e >= (1400u << 20)) & !zero) q = plain_div(a, b);
+  return q;
+}
+// x / dxy of the FP64 state. Out of line for the same reason; at a spacing of
+// 3, 1000 x 700 cells took 131 us a step with plain divisions, 112 us so.
+__device__ __noinline__ double over_dxy(double x, double dxy, double inv) { return over(x, dxy, inv); }
+__device__ __forceinline__ double div_dxy(const fx_dev& d, double x) {
+  return d.dxy_pow2 ? x * d.inv_dxy : over_dxy(x, d.dxy, d.inv_dxy);
+}
+constexpr double DAY_MM = 1000. * 3600. * 24.;  // mm/day to m/s
+
+// max(x, c) for a c that is a number, by a compare and a select: the bits of
+// fmax (an x that is no number gives c, and max(-0, 0) is 0), which takes a
+// few instructions more.
+__device__ __forceinline__ double at_least(double x, double c) { return x > c ? x : c; }
+__device__ __forceinline__ double max0(double x) { return at_least(x, 0.0); }
+
+// The edge weir's flux (solver_wetdomain.cpp:302-307): out of line, only edge
+// cells of the domain have one.
+__device__ __noinline__ double edge_weir(double volrat, double sqrt_g, double hp) {
+  return fmin(volrat, sqrt_g * fx_pow15(fmax(hp, 0.0)));
+}
+
 // Cube root of x >= 0 by Newton iteration on the mantissa, using only
 // frexp/ldexp and IEEE +,-,*,/, so the oracle's C (ox_cbrt) computes the
 // same bits. Used by the Manning extension only.
@@ -98,8 +157,28 @@ __device__ __forceinline__ double fx_cbrt(double x) {
   e -= r;
   double y = 0.5 + 0.35 * m;
 #pragma unroll 1
-  for (int i = 0; i < 7; ++i) y = y - (y * y * y - m) / (3.0 * y * y);
+  for (int i = 0; i < 7; ++i) {
+    y = y - (y * y * y - m) / (3.0 * y * y);
+  }
   return ldexp(y, e / 3);
+}
+
+// The stencil cells a thread reads, in two passes without an integer division: warp
+// ly reads column ly, then warps 0 and 1 the last two columns and the others
+// the two rows beyond the warp's 32. False: none in this pass.
+template <int BY>
+__device__ __forceinline__ bool stencil_cell(int pass, int lx, int ly, int& sr, int& sc) {
+  sr = lx;
+  sc = ly;
+  if (pass == 0) return true;
+  if (ly < 2) {
+    sc = BY + ly;
+    return true;
+  }
+  const int e = (ly - 2) * BX + lx;
+  sr = BX + (e & 1);
+  sc = e >> 1;
+  return e < 2 * Tile<BY>::SY;
 }
 
 __device__ __forceinline__ int sidx(int sr, int sc) { return sc * SX + sr; }
@@ -107,20 +186,19 @@ __device__ __forceinline__ int sidx(int sr, int sc) { return sc * SX + sr; }
 // solver_wetdomain.cpp:27-342 for the flux cell at stencil (sr, sc).
 template <class SM>
 __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
-                           double dtl, double out[6]) {
+                           Over dt, double out[6]) {
   const double hdryl = d.hdry, gaccl = d.gaccl;
   const int P = sidx(sr, sc), W = sidx(sr - 1, sc), E = sidx(sr + 1, sc);
   const int Sx = sidx(sr, sc - 1), N = sidx(sr, sc + 1);
   const int ES = sidx(sr + 1, sc - 1), EN = sidx(sr + 1, sc + 1), WN = sidx(sr - 1, sc + 1);
   auto ksat = [&](int k) { return (S.cls[k] & C_INT) ? d.ks : 0.0; };
-  auto hat = [&](int k) { return fmax(0.0, S.z[k] - S.zb[k]); };
+  auto hat = [&](int k) { return max0(S.z[k] - S.zb[k]); };
   const double kspl = ksat(P);
   const double nueml = d.nueml, cvdefl = d.cvdefl;
   const unsigned dx = d.dxy_u, dy = d.dxy_u;
   bool lroe = true;
   double volrat = d.volrat_mode == 0 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0;
 
-  const bool ldp_dry = S.cls[P] & C_DRY;
   const bool lde_dry = S.cls[E] & C_DRY;
   const bool ldn_dry = S.cls[N] & C_DRY;
 
@@ -131,12 +209,11 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
 
   const double zbpe = .5 * (zbe + zbp);
   const double zbpn = .5 * (zbn + zbp);
-  const double hp = fmax(0.0, zp - zbp);
-  const double hp0 = fmax(fmax(hdryl, hp), kspl);
-  const double hw = fmax(0.0, zw - zbw);
-  double he = fmax(0.0, ze - zbe);
-  const double hs = fmax(0.0, zs - zbs);
-  double hn = fmax(0.0, zn - zbn);
+  const double hp = max0(zp - zbp);
+  const double hw = max0(zw - zbw);
+  double he = max0(ze - zbe);
+  const double hs = max0(zs - zbs);
+  double hn = max0(zn - zbn);
 
   double hme = .5 * (hp + he);
   double qme = .5 * (qp + qe);
@@ -153,7 +230,7 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
   const double dqn = qn - qp;
 
   if (lde_dry) {  // :121-147
-    hme = fmax(0.0, zp - zbpe);
+    hme = max0(zp - zbpe);
     he = 0.0;
     qe = 0.0;
     re = 0.0;
@@ -164,7 +241,7 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
       } else {
         dze = fmin(fabs(dze), hme);
         qme = 0.296 * dze * sqrt(gaccl * dze);
-        volrat = 0.5 * dx * hp / dtl;
+        volrat = dt.of(0.5 * dx * hp);
         qme = fmin(qme, volrat);
         rme = 0.0;
       }
@@ -176,7 +253,7 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
     lroe = false;
   }
   if (ldn_dry) {  // :148-175
-    hmn = fmax(0.0, zp - zbpn);
+    hmn = max0(zp - zbpn);
     hn = 0.0;
     qn = 0.0;
     rn = 0.0;
@@ -188,7 +265,7 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
         dzn = fmin(fabs(dzn), hmn);
         rmn = 0.296 * dzn * sqrt(gaccl * dzn);
         qmn = 0.0;
-        volrat = 0.5 * dy * hp / dtl;
+        volrat = dt.of(0.5 * dy * hp);
         rmn = fmin(rmn, volrat);
       }
     } else {
@@ -203,22 +280,24 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
   // the reference (set to 0 by initiate.cpp:176 and both update loops).
   const double cme = sqrt(gaccl * hme);
   const double cmn = sqrt(gaccl * hmn);
-  const double ume = qme / fmax(hme, hdryl);
-  const double vme = rme / fmax(hme, hdryl);
-  const double umn = qmn / fmax(hmn, hdryl);
-  const double vmn = rmn / fmax(hmn, hdryl);
+  const Over he_(at_least(hme, hdryl)), hn_(at_least(hmn, hdryl));
+  const double ume = he_.of(qme);
+  const double vme = he_.of(rme);
+  const double umn = hn_.of(qmn);
+  const double vmn = hn_.of(rmn);
   const double cnp = cvdefl * 0.0 * hp + nueml;
   const double cne = cvdefl * 0.0 * he + nueml;
   const double cnn = cvdefl * 0.0 * hn + nueml;
   const double hne = .5 * (cnp + cne) * sqrt(hp * he);
   const double hnn = .5 * (cnp + cnn) * sqrt(hp * hn);
 
-  const double up = qp / hp0;
   // neighbour velocities from the stencil (solver_wetdomain.cpp: each is
   // q / max(max(h, hdry), ks) of its cell; a dry neighbour's discharge is 0,
   // so its velocity is 0 whatever depth the division uses)
-  double un, us0, use0, une, ve, vw, vwn, ven;
+  double up, vp, un, us0, use0, une, ve, vw, vwn, ven;
   if constexpr (SM::VEL) {
+    up = S.u[P];
+    vp = S.v[P];
     un = S.u[N];
     us0 = S.u[Sx];
     use0 = S.u[ES];
@@ -228,6 +307,9 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
     vwn = S.v[WN];
     ven = S.v[EN];
   } else {
+    const Over hp_(fmax(fmax(hdryl, hp), ksat(P)));
+    up = hp_.of(qp);
+    vp = hp_.of(rp);
     un = qn / fmax(fmax(hn, hdryl), ksat(N));
     us0 = S.qx[Sx] / fmax(fmax(hs, hdryl), ksat(Sx));
     use0 = S.qx[ES] / fmax(fmax(hat(ES), hdryl), ksat(ES));
@@ -237,11 +319,9 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
     vwn = S.qy[WN] / fmax(fmax(hat(WN), hdryl), ksat(WN));
     ven = S.qy[EN] / fmax(fmax(hat(EN), hdryl), ksat(EN));
   }
-  const double vp = rp / hp0;
 
-
-  const double txye = hne * (fx_div_dxy(d, ve - vp) + fx_div_dxy(d, .25 * (un + une - us0 - use0)));
-  const double txyn = hnn * (fx_div_dxy(d, un - up) + fx_div_dxy(d, .25 * (ve + ven - vw - vwn)));
+  const double txye = hne * (div_dxy(d, ve - vp) + div_dxy(d, .25 * (un + une - us0 - use0)));
+  const double txyn = hnn * (div_dxy(d, un - up) + div_dxy(d, .25 * (ve + ven - vw - vwn)));
 
   const double fe1c = qme;
   const double fe2c = qme * ume;
@@ -277,7 +357,7 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
     fe2r = -(a21 * dze + a22 * dqe) * cc;
     fe3r = -(a31 * dze + a32 * dqe + a33 * dre) * cc;
 
-    if (!ldp_dry && hmn > d.hdry) {
+    if (hmn > d.hdry) {  // this cell is wet (ldp == 0)
       double dzna = fabs(dzn);
       double dhna = fabs(hn - hp);
       dzna = fmin(dzna, dhna);
@@ -315,22 +395,22 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
   const double fn2 = fn2c + fn2r;
   const double fn3 = fn3c + fn3r + fn3p;
 
-  if (icol == 1 || icol == d.nc) fn1 = fmin(volrat, d.sqrt_gaccl * fx_pow15(fmax(hp, 0.0)));
-  if (irow == 1 || irow == d.nr) fe1 = fmin(volrat, d.sqrt_gaccl * fx_pow15(fmax(hp, 0.0)));
+  if (icol == 1 || icol == d.nc) fn1 = edge_weir(volrat, d.sqrt_gaccl, hp);
+  if (irow == 1 || irow == d.nr) fe1 = edge_weir(volrat, d.sqrt_gaccl, hp);
 
   const double volpot = d.arbase * hp;
-  volrat = volpot / dtl;
+  volrat = dt.of(volpot);
   if (volrat > 0.0) {  // :309-332
-    if (fe1 > 0.0 && fn1 > 0.0) {
+    if ((fe1 > 0.0) & (fn1 > 0.0)) {
       if (fe1 * dy + fn1 * dx > volrat) {
         double cf = fn1 * dx / (fe1 * dy + fn1 * dx);
-        fe1 = fx_div_dxy(d, (1. - cf) * volrat);
-        fn1 = fx_div_dxy(d, cf * volrat);
+        fe1 = div_dxy(d, (1. - cf) * volrat);
+        fn1 = div_dxy(d, cf * volrat);
       }
     } else if (fe1 > 0.0) {
-      fe1 = fx_div_dxy(d, fmin(fe1 * dy, volrat));
+      fe1 = div_dxy(d, fmin(fe1 * dy, volrat));
     } else if (fn1 > 0.0) {
-      fn1 = fx_div_dxy(d, fmin(fn1 * dx, volrat));
+      fn1 = div_dxy(d, fmin(fn1 * dx, volrat));
     }
   } else {
     fe1 = 0.0;
@@ -403,8 +483,8 @@ __device__ void solver_dry(const fx_dev& d, const SM& S, int sr, int sc, int iro
       }
     }
   }
-  if (icol == 1 || icol == d.nc) fn1 = fmin(volrat, d.sqrt_gaccl * fx_pow15(fmax(hp, 0.0)));
-  if (irow == 1 || irow == d.nr) fe1 = fmin(volrat, d.sqrt_gaccl * fx_pow15(fmax(hp, 0.0)));
+  if (icol == 1 || icol == d.nc) fn1 = edge_weir(volrat, d.sqrt_gaccl, hp);
+  if (irow == 1 || irow == d.nr) fe1 = edge_weir(volrat, d.sqrt_gaccl, hp);
   out[0] = fe1;
   out[1] = fe2;
   out[2] = fe3;
@@ -414,15 +494,15 @@ __device__ void solver_dry(const fx_dev& d, const SM& S, int sr, int sc, int iro
 }
 
 // The Courant candidate of one cell (main.cpp:308-316), or +inf if dry.
-__device__ __forceinline__ void courant_cell(const fx_dev& d, double h, double qx, double qy,
-                                             double& dtc, double& hm) {
+__device__ __forceinline__ void courant_cell(const fx_dev& d, double h, double qx, double qy, double& dtc,
+                                             double& hm) {
   dtc = __longlong_as_double(0x7ff0000000000000LL);
   hm = 0.0;
   if (h > d.hdry) {
-    double hp = fmax(h, d.hdry);
     double c0 = sqrt(d.gaccl * h);
-    double u0 = fmax(.000001, fabs(qx / hp));
-    double v0 = fmax(.000001, fabs(qy / hp));
+    const Over hp(h);  // max(h, hdry) is h here
+    double u0 = fmax(.000001, fabs(hp.of(qx)));
+    double v0 = fmax(.000001, fabs(hp.of(qy)));
     // min(a / (u0 + c0), a / (v0 + c0)) with a > 0 is a / (max(u0, v0) + c0)
     // bit for bit: rounded addition and division are monotone
     double c = d.cfl_dxy / (fmax(u0, v0) + c0);
@@ -497,6 +577,8 @@ __device__ __forceinline__ StageOff stage_off(int bx) {
 // the largest wet depth (exact in any order) and the FP64 water budget.
 struct TilePart {
   double dtc, hm, melt, out;
+  float hmf;       // FP32 state: high part of hm
+  unsigned speed;  // largest approximate wave speed (float bits) whose Courant candidate is in dtc, the warp's
   __device__ __forceinline__ void add(double dt, double h, double m, double o) {
     dtc = fmin(dtc, dt);
     hm = fmax(hm, h);
@@ -508,6 +590,8 @@ __device__ __forceinline__ TilePart tile_part() {
   TilePart p;
   p.dtc = __longlong_as_double(0x7ff0000000000000LL);
   p.hm = p.melt = p.out = 0.0;
+  p.hmf = 0.0f;
+  p.speed = 0u;
   return p;
 }
 
@@ -515,9 +599,36 @@ __device__ __forceinline__ TilePart tile_part() {
 struct StepCtl {
   double dtfl, meteoi, meteo_rate, mconc, inflowi;
   double twet_inc;  // dtfl / 3600, the wet-time increment (hydrodynamics_calc.cpp:69-70), once per tile
+  Over dt;          // quotients over dtfl, FP64 state
+  float dtf, twet_f;  // dtfl and twet_inc in FP32
+  // Slot planes (fx_slot) of the state after the previous step and of the one
+  // this step writes, and the same of the two-plane fields (fx_pp): here, once
+  // per block, because the slot is a 64-bit remainder (the FP32 kernel at
+  // 4096 x 4096 cells 1.11 ms a step with it in every tile and with stencil
+  // indices by division, 1.02 ms without)
+  long long sprev, scur, pprev, pcur;
   long long steps;
   int live, active;
 };
+__device__ __forceinline__ void read_ctl(const fx_dev& d, StepCtl& c) {
+  const fx_ctl& g = *d.ctl;
+  c.dtfl = g.dtfl;
+  c.meteoi = g.meteoi;
+  c.meteo_rate = g.meteo_rate;
+  c.mconc = g.mconc;
+  c.inflowi = g.inflowi;
+  c.twet_inc = g.dtfl / 3600;
+  c.dt = Over(g.dtfl);
+  c.dtf = (float)g.dtfl;
+  c.twet_f = (float)c.twet_inc;
+  c.sprev = fx_slot(d, g.steps - 1);
+  c.scur = fx_slot(d, g.steps);
+  c.pprev = fx_pp(d, g.steps - 1);
+  c.pcur = fx_pp(d, g.steps);
+  c.steps = g.steps;
+  c.live = g.live;
+  c.active = g.active;
+}
 
 // Block sum of the step's water budget terms, one double atomic each.
 __device__ void reduce_budget(const fx_dev& d, double* red, double melt, double out) {
@@ -553,7 +664,7 @@ __device__ __forceinline__ void reduce_part(const fx_dev& d, SM& S, const TilePa
 }
 
 __device__ __forceinline__ double melt_depth(const fx_dev& d, const StepCtl& c, long long gi) {
-  if (d.melt_mult) return (double)c.meteo_rate * d.melt_mult[gi] / (1000. * 3600. * 24.) * c.dtfl;
+  if (d.melt_mult) return over((double)c.meteo_rate * d.melt_mult[gi], DAY_MM, 1.0 / DAY_MM) * c.dtfl;
   if (d.melt_mult_f) return (double)c.meteo_rate * (double)d.melt_mult_f[gi] / (1000. * 3600. * 24.) * c.dtfl;
   return c.meteoi;
 }
@@ -606,6 +717,7 @@ struct HydroSmem32 {
   // cell for the wet solver's shear terms (each face reads eight of them)
   static constexpr bool VEL = true;
   float u[NSTEN], v[NSTEN];
+  float mi[NSTEN];  // the step's melt depth, of the cells that take it
   float f[6][NFLUX];
   unsigned char cls[NSTEN];
 };
@@ -669,8 +781,39 @@ __device__ __forceinline__ void courant_cell32(const fx_dev& d, double depth, fl
   }
 }
 
+// The Courant candidates and depths of a warp's cells into its partials. The
+// step's dt needs only the smallest candidate, cfl dxy / speed, so a cell
+// whose approximate speed (relative error below 2^-18: two approximate
+// operations and a handful of roundings on FP32 operands) is more than 2^-15
+// below one whose candidate is in the partials already cannot be the
+// smallest, and its two FP64 divisions and root are skipped: a warp evaluates
+// its first cells and then the few that set a record. The same for the FP64
+// depth, by its high part. The results are those of evaluating every cell.
+__device__ __forceinline__ void courant_tile32(const fx_dev& d, bool wet, float eta, float lo, float qx, float qy,
+                                               TilePart& acc) {
+  float speed = 0.0f;
+  if (wet) {
+    float r, s;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(eta));
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(d.f.gaccl * eta));
+    speed = fmaxf(.000001f, fmaxf(fabsf(qx), fabsf(qy)) * r) + s;
+    if (eta >= acc.hmf) {
+      acc.hm = fmax(acc.hm, fx_dd_val(eta, lo));
+      acc.hmf = eta;
+    }
+  }
+  const bool odd = !(speed < 1e30f);  // an overflow or a NaN bounds nothing
+  const unsigned bits = odd ? 0u : __float_as_uint(speed);
+  acc.speed = max(acc.speed, __reduce_max_sync(0xffffffffu, bits));
+  if (wet && (odd || speed >= __uint_as_float(acc.speed) * (1.0f - 0x1p-15f))) {
+    double dtc, hm;
+    courant_cell32(d, fmax(0.0, fx_dd_val(eta, lo)), qx, qy, dtc, hm);
+    acc.dtc = fmin(acc.dtc, dtc);
+  }
+}
+
 __device__ __forceinline__ float div_dxy_f(const fx_dev& d, float x) {
-  return d.dxy_pow2 ? x * (float)d.inv_dxy : fdiv(x, (float)d.dxy);
+  return d.dxy_pow2 ? x * d.f.inv_dxy : fdiv(x, d.f.dxy);
 }
 
 // The Roe face-depth test of the FP32 state, `.5 * (max(0, dP) + max(0, dQ))
@@ -688,19 +831,31 @@ __device__ __forceinline__ bool above_hdry(float x, float lo, float hi, F exact)
   return exact();
 }
 
+// The compensated depth eta + lo against hdry, decided from eta where that is
+// safe (|lo| is at most half an ulp of eta, so the same band serves).
+__device__ __forceinline__ bool dd_le_hdry(const fx_dev& d, float eta, float lo) {
+  if (eta > d.f.hdry_hi) return false;
+  if (eta < d.f.hdry_lo) return true;
+  return fx_dd_val(eta, lo) <= d.hdry;
+}
+__device__ __forceinline__ bool dd_lt_hdry(const fx_dev& d, float eta, float lo) {
+  if (eta > d.f.hdry_hi) return false;
+  if (eta < d.f.hdry_lo) return true;
+  return fx_dd_val(eta, lo) < d.hdry;
+}
+
 template <class SM>
 __device__ void solver_wet32(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
                              float dtl, float out[6]) {
   const double hdry = d.hdry;
-  const float hdryl = (float)d.hdry, gaccl = (float)d.gaccl;
-  const float hdry_lo = (float)(hdry * (1.0 - 0x1p-19)), hdry_hi = (float)(hdry * (1.0 + 0x1p-19));
+  const float hdryl = d.f.hdry, gaccl = d.f.gaccl, hdry_lo = d.f.hdry_lo, hdry_hi = d.f.hdry_hi;
   const int P = sidx(sr, sc), W = sidx(sr - 1, sc), E = sidx(sr + 1, sc);
   const int Sx = sidx(sr, sc - 1), N = sidx(sr, sc + 1);
   const int ES = sidx(sr + 1, sc - 1), EN = sidx(sr + 1, sc + 1), WN = sidx(sr - 1, sc + 1);
-  auto ksat = [&](int k) { return (S.cls[k] & C_INT) ? (float)d.ks : 0.0f; };
+  auto ksat = [&](int k) { return (S.cls[k] & C_INT) ? d.f.ks : 0.0f; };
   const float kspl = ksat(P);
-  const float nueml = (float)d.nueml;
-  const float dx = (float)d.dxy, dy = dx;
+  const float nueml = d.f.nueml;
+  const float dx = d.f.dxy, dy = dx;
   bool lroe = true;
   float volrat = d.volrat_mode == 0 ? __int_as_float(0x7f800000) : 0.0f;
   const bool ldp_dry = S.cls[P] & C_DRY, lde_dry = S.cls[E] & C_DRY, ldn_dry = S.cls[N] & C_DRY;
@@ -834,17 +989,17 @@ __device__ void solver_wet32(const fx_dev& d, const SM& S, int sr, int sc, int i
     if (icol == 1 || icol == d.nc) fn1 = fminf(volrat, weir);
     if (irow == 1 || irow == d.nr) fe1 = fminf(volrat, weir);
   }
-  volrat = fdiv((float)d.arbase * hp, dtl);
+  volrat = fdiv(d.f.area * hp, dtl);
   {  // solver_wetdomain.cpp:309-332 as selects: one straight-line block, the
      // quotient of the split kept only when the split applies
     const float sdy = fe1 * dy, sdx = fn1 * dx, sum = sdy + sdx;
     const bool pos = volrat > 0.0f, pe = fe1 > 0.0f, pn = fn1 > 0.0f;
-    const bool split = pos && pe && pn && sum > volrat;
+    const bool split = pos & pe & pn & (sum > volrat);
     const float cf = fdiv(sdx, split ? sum : 1.0f);
     const float e = div_dxy_f(d, split ? (1.f - cf) * volrat : fminf(sdy, volrat));
     const float n = div_dxy_f(d, split ? cf * volrat : fminf(sdx, volrat));
-    fe1 = !pos ? 0.0f : ((split || (pe && !pn)) ? e : fe1);
-    fn1 = !pos ? 0.0f : ((split || (pn && !pe)) ? n : fn1);
+    fe1 = !pos ? 0.0f : ((split | (pe & !pn)) ? e : fe1);
+    fn1 = !pos ? 0.0f : ((split | (pn & !pe)) ? n : fn1);
   }
   out[0] = fe1;
   out[1] = fe2;
@@ -858,7 +1013,7 @@ template <class SM>
 __device__ void solver_dry32(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
                              float dtl, float out[6]) {
   const int P = sidx(sr, sc), E = sidx(sr + 1, sc), N = sidx(sr, sc + 1);
-  const float gaccl = (float)d.gaccl;
+  const float gaccl = d.f.gaccl;
   float volrat = d.volrat_mode == 0 ? __int_as_float(0x7f800000) : 0.0f;
   const bool lde_dry = S.cls[E] & C_DRY, ldn_dry = S.cls[N] & C_DRY;
   const double sx_d = S.zb[E] - S.zb[P], sy_d = S.zb[N] - S.zb[P];
@@ -878,7 +1033,7 @@ __device__ void solver_dry32(const fx_dev& d, const SM& S, int sr, int sc, int i
         // the surface difference is positive (decided in FP64); its FP32
         // value can round to 0, where the inflow and its momentum are 0
         dze = fminf((float)dze_d, hme);
-        volrat = fdiv((float)d.dxy * he, dtl);
+        volrat = fdiv(d.f.dxy * he, dtl);
         if (dze > 0.0f) {
           float qme = 0.296f * dze * fsqrt(gaccl * dze);
           hme = 0.444f * dze;
@@ -897,7 +1052,7 @@ __device__ void solver_dry32(const fx_dev& d, const SM& S, int sr, int sc, int i
         fn3 = .5f * gaccl * hmn * hmn;
       } else {
         dzn = fminf((float)dzn_d, hmn);
-        volrat = fdiv((float)d.dxy * hn, dtl);
+        volrat = fdiv(d.f.dxy * hn, dtl);
         if (dzn > 0.0f) {
           float rmn = 0.296f * dzn * fsqrt(gaccl * dzn);
           hmn = 0.444f * dzn;
@@ -950,10 +1105,9 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
   const int irow0 = 1 + tile.bx * TX, icol0 = 1 + tile.by * TY;
   const int irow = irow0 + lx, icol = icol0 + ly;
   const bool own = lx < TX && ly < TY && irow <= d.nr && icol <= d.nc;
-  const float dtl = (float)c.dtfl;
+  const float dtl = c.dtf;
   const bool melt_on = d.has_meteo != 0;
-  const long long sprev = fx_slot(d, c.steps - 1), scur = fx_slot(d, c.steps);
-  const long long pprev = fx_pp(d, c.steps - 1), pcur = fx_pp(d, c.steps);
+  const long long sprev = c.sprev, scur = c.scur, pprev = c.pprev, pcur = c.pcur;
   double dtc = __longlong_as_double(0x7ff0000000000000LL), hm = 0.0, bmelt = 0.0, bout = 0.0;
 
   if (!c.active) {
@@ -1012,8 +1166,11 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     const float* g_qy = reinterpret_cast<const float*>(stg + L::O_QY);
     const float* g_mm = reinterpret_cast<const float*>(stg + L::O_MM);
     const uint8_t* g_fl = stg + L::O_FL;
-    for (int k = tid; k < NSTEN; k += NTHREADS) {
-      const int sr = k % SX, scc = k / SX;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      int sr, scc;
+      if (!stencil_cell<BY>(pass, lx, ly, sr, scc)) break;
+      const int k = sidx(sr, scc);
       const int r = irow0 - 2 + sr, q = icol0 - 2 + scc;
       const int i4 = scc * STG_W4 + sr + so.o4;
       float eta = g_eta[i4], lo = g_lo[i4], qx = g_qx[i4], qy = g_qy[i4];
@@ -1023,9 +1180,13 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
         cl = C_INT;
         const uint8_t fl = g_fl[scc * STG_W1 + sr + so.o1];
         if (fl & FX_F_WALL) cl |= C_WALL;
-        if (melt_on && !(fl & FX_F_NODATA)) fx_dd_add(eta, lo, melt32(d, c, g_mm[i4]));
+        if (melt_on && !(fl & FX_F_NODATA)) {
+          const float mi = melt32(d, c, g_mm[i4]);
+          S.mi[k] = mi;
+          fx_dd_add(eta, lo, mi);
+        }
         if (is_inflow(d, r, q)) inflow_eta(eta, lo, c.inflowi);
-        if (fx_dd_val(eta, lo) <= d.hdry) {
+        if (dd_le_hdry(d, eta, lo)) {
           qx = 0.f;
           qy = 0.f;
           cl |= C_DRY;
@@ -1038,14 +1199,17 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       S.qy[k] = qy;
       S.cls[k] = cl;
       {
-        const float den = fmaxf(fmaxf(fmaxf(0.0f, eta), (float)d.hdry), (cl & C_INT) ? (float)d.ks : 0.0f);
+        const float den = fmaxf(fmaxf(fmaxf(0.0f, eta), d.f.hdry), (cl & C_INT) ? d.f.ks : 0.0f);
         S.u[k] = fdiv(qx, den);
         S.v[k] = fdiv(qy, den);
       }
     }
   } else
-  for (int k = tid; k < NSTEN; k += NTHREADS) {
-    const int sr = k % SX, scc = k / SX;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    int sr, scc;
+    if (!stencil_cell<BY>(pass, lx, ly, sr, scc)) break;
+    const int k = sidx(sr, scc);
     const int r = irow0 - 2 + sr, q = icol0 - 2 + scc;
     float eta = 0.f, lo = 0.f, qx = 0.f, qy = 0.f;
     double zb = 0.0;
@@ -1061,9 +1225,13 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
         cl = C_INT;
         const uint8_t fl = d.flags[sprev + gi];
         if (fl & FX_F_WALL) cl |= C_WALL;
-        if (melt_on && !(fl & FX_F_NODATA)) fx_dd_add(eta, lo, melt32(d, c, d.melt_mult_f ? d.melt_mult_f[gi] : 1.0f));
+        if (melt_on && !(fl & FX_F_NODATA)) {
+          const float mi = melt32(d, c, d.melt_mult_f ? d.melt_mult_f[gi] : 1.0f);
+          S.mi[k] = mi;
+          fx_dd_add(eta, lo, mi);
+        }
         if (is_inflow(d, r, q)) inflow_eta(eta, lo, c.inflowi);
-        if (fx_dd_val(eta, lo) <= d.hdry) {
+        if (dd_le_hdry(d, eta, lo)) {
           qx = 0.f;
           qy = 0.f;
           cl |= C_DRY;
@@ -1077,7 +1245,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     S.qy[k] = qy;
     S.cls[k] = cl;
       {
-        const float den = fmaxf(fmaxf(fmaxf(0.0f, eta), (float)d.hdry), (cl & C_INT) ? (float)d.ks : 0.0f);
+        const float den = fmaxf(fmaxf(fmaxf(0.0f, eta), d.f.hdry), (cl & C_INT) ? d.f.ks : 0.0f);
         S.u[k] = fdiv(qx, den);
         S.v[k] = fdiv(qy, den);
       }
@@ -1087,19 +1255,18 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
   if (__syncthreads_or(bad)) return false;
   {
     // Each thread computes its own face-flux cell (NFLUX == NTHREADS), wet,
-    // dry or kept, without the FP64 path's work lists: in FP32 the lists'
-    // gathering cost more than the divergence they avoid (4096^2 wet start
-    // 1.4 % and the 64-scenario batch 6 % faster without them).
-    const int k = tid;
-    const int fr = k % FXN, fc = k / FXN;
+    // dry or kept: gathering each kind's cells in lists cost more than the
+    // divergence it avoids (4096^2 wet start 1.4 % and the 64-scenario batch
+    // 6 % faster without).
+    const int k = tid, fr = lx, fc = ly;
     const int sr = fr + 1, scc = fc + 1;
     const unsigned char cl = S.cls[sidx(sr, scc)];
     float o[6];
     if (!(cl & C_INT) || (cl & C_WALL)) {
       for (int j = 0; j < 6; ++j) S.f[j][k] = 0.0f;
     } else if (cl & C_DRY) {
-      const bool alldry = (S.cls[sidx(sr - 1, scc)] & C_DRY) && (S.cls[sidx(sr + 1, scc)] & C_DRY) &&
-                          (S.cls[sidx(sr, scc - 1)] & C_DRY) && (S.cls[sidx(sr, scc + 1)] & C_DRY);
+      const bool alldry = S.cls[sidx(sr - 1, scc)] & S.cls[sidx(sr + 1, scc)] & S.cls[sidx(sr, scc - 1)] &
+                          S.cls[sidx(sr, scc + 1)] & C_DRY;
       if (alldry) {  // all five cells dry: the last computed fluxes stay (solver_drydomain.cpp:60-76)
         const long long gi = fx_ix(d, irow0 - 1 + fr, icol0 - 1 + fc);
         const float* rp = fx_rec(d, sprev + gi);
@@ -1119,6 +1286,8 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     }
   }
   __syncthreads();
+  bool wet = false;
+  float c_eta = 0.f, c_lo = 0.f, c_qx = 0.f, c_qy = 0.f;  // this thread's cell after the update
   if (own) {
     const long long gi = fx_ix(d, irow, icol);
     const int sP = sidx(lx + 2, ly + 2);
@@ -1135,9 +1304,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     if (melt_on && !(fl & FX_F_NODATA)) {
       h0v = fmaxf(eta1, 0.0f);
       hpv = fmaxf(etapre, 0.0f);
-      const float mm = !d.melt_mult_f ? 1.0f
-                       : (stg ? reinterpret_cast<const float*>(stg + L::O_MM)[i4] : d.melt_mult_f[gi]);
-      miv = melt32(d, c, mm);
+      miv = S.mi[sP];
       mi = (double)miv;
       bmelt = mi * d.arbase;
     }
@@ -1149,7 +1316,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       bmelt += (fx_dd_val(eta1, S.eta_lo[sP]) - dm) * d.arbase;
       h0v = fmaxf(eta1, 0.0f);
     }
-    if (!(cl & C_DRY)) d.twet_f[gi] += (float)c.twet_inc;
+    if (!(cl & C_DRY)) d.twet_f[gi] += c.twet_f;
     float dh = 0.f, dqx = 0.f, dqy = 0.f, qxfP = 0.f, qyfP = 0.f;
     if (!wall) {
       dh = (div_dxy_f(d, S.f[0][fW] - S.f[0][fP]) + div_dxy_f(d, S.f[3][fS] - S.f[3][fP])) * dtl;
@@ -1162,15 +1329,14 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       if (icol == d.nc || (clN & C_WALL)) bout += (double)S.f[3][fP] * d.dxy * c.dtfl;
     }
     const unsigned char clW = S.cls[sidx(lx + 1, ly + 2)], clS = S.cls[sidx(lx + 2, ly + 1)];
-    const float qxfW = ((clW & C_INT) && !(clW & C_WALL)) ? S.f[0][fW] * dtl : 0.0f;
-    const float qyfS = ((clS & C_INT) && !(clS & C_WALL)) ? S.f[3][fS] * dtl : 0.0f;
+    const float qxfW = ((clW & (C_INT | C_WALL)) == C_INT) ? S.f[0][fW] * dtl : 0.0f;
+    const float qyfS = ((clS & (C_INT | C_WALL)) == C_INT) ? S.f[3][fS] * dtl : 0.0f;
     float eta = eta1, lo = S.eta_lo[sP];
     fx_dd_add(eta, lo, dh);
     const float h = fmaxf(0.0f, eta);
-    const double depth = fx_dd_val(eta, lo);
     float qx, qy;
     uint8_t ld;
-    if (depth < d.hdry || wall) {
+    if (dd_lt_hdry(d, eta, lo) || wall) {
       qx = qy = 0.0f;
       ld = 1;
     } else {
@@ -1184,7 +1350,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       const float n = d.manning_f[gi];
       if (n != 0.0f) {
         const float qm = fsqrt(qx * qx + qy * qy);
-        const float den = 1.0f + fdiv(dtl * (float)d.gaccl * n * n * qm, h * h * fcbrt(h));
+        const float den = 1.0f + fdiv(dtl * d.f.gaccl * n * n * qm, h * h * fcbrt(h));
         const float rden = frcp(den);
         qx = qx * rden;
         qy = qy * rden;
@@ -1199,11 +1365,11 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     float fe1v = 0.0f, fn1v = 0.0f;
     if ((cl & C_INT) && !wall) {
       const bool computed =
-          !(cl & C_DRY) || !((S.cls[sidx(lx + 1, ly + 2)] & C_DRY) && (S.cls[sidx(lx + 3, ly + 2)] & C_DRY) &&
-                             (S.cls[sidx(lx + 2, ly + 1)] & C_DRY) && (S.cls[sidx(lx + 2, ly + 3)] & C_DRY));
+          !(cl & C_DRY) || !(S.cls[sidx(lx + 1, ly + 2)] & S.cls[sidx(lx + 3, ly + 2)] &
+                              S.cls[sidx(lx + 2, ly + 1)] & S.cls[sidx(lx + 2, ly + 3)] & C_DRY);
       fe1v = S.f[0][fP];
       fn1v = S.f[3][fP];
-      if (computed && (d.store_all_fluxes || !(depth > d.hdry))) {
+      if (computed && (d.store_all_fluxes || dd_le_hdry(d, eta, lo))) {
         d.fe2_f[gi] = S.f[1][fP];
         d.fe3_f[gi] = S.f[2][fP];
         d.fn2_f[gi] = S.f[4][fP];
@@ -1211,9 +1377,15 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       }
     }
     put_rec32(d, scur + gi, h0v, h, hpv, miv, fe1v, fn1v, fl1);
-    courant_cell32(d, fmax(0.0, depth), qx, qy, dtc, hm);
+    wet = eta > 0.0f && !dd_le_hdry(d, eta, lo);
+    c_eta = eta;
+    c_lo = lo;
+    c_qx = qx;
+    c_qy = qy;
   }
-  acc.add(dtc, hm, bmelt, bout);
+  courant_tile32(d, wet, c_eta, c_lo, c_qx, c_qy, acc);
+  acc.melt += bmelt;
+  acc.out += bout;
   return true;
 }
 
@@ -1238,8 +1410,7 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   // writes (h, h0, fe_1, fn_1, flags), and the two planes of z, qx, qy (see
   // fx_common.cuh): every block reads the previous step's plane, halo
   // included, and writes the other.
-  const long long sprev = fx_slot(d, c.steps - 1), scur = fx_slot(d, c.steps);
-  const long long pprev = fx_pp(d, c.steps - 1), pcur = fx_pp(d, c.steps);
+  const long long sprev = c.sprev, scur = c.scur, pprev = c.pprev, pcur = c.pcur;
 
   if (!c.active) {
     // No wet cell: the step is the Courant scan plus add_meteo only
@@ -1250,22 +1421,22 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       const long long gi = fx_ix(d, irow, icol);
       const double zb = d.zb[gi], zpre = d.z[pprev + gi];
       const uint8_t fl = d.flags[sprev + gi];
-      const double hpre = fmax(0.0, zpre - zb);
+      const double hpre = max0(zpre - zb);
       uint8_t ld = hpre > d.hdry ? 0 : 1;  // Courant scan (:308-320)
       double z1 = zpre, h1 = hpre, hpv = 0.0;
       if (melt_on && zb != d.nodata) {
         const double mi = melt_depth(d, c, gi);
         bmelt = mi * d.arbase;
-        hpv = fmax(zpre - zb, 0.0);  // the dilution's hp (common.cpp:216)
+        hpv = max0(zpre - zb);  // the dilution's hp (common.cpp:216)
         z1 = zpre + mi;
-        h1 = fmax(z1 - zb, 0.0);
+        h1 = max0(z1 - zb);
         if (h1 <= d.hdry) ld = 0;  // common.cpp:219-222
       }
       if (is_inflow(d, irow, icol)) {  // common.cpp:300-315
         const double zm = z1;
-        record_inflow_hm(d, c, fmax(zm - zb, 0.0));
+        record_inflow_hm(d, c, max0(zm - zb));
         z1 = inflow_z(z1, zb, c.inflowi);
-        h1 = fmax(z1 - zb, 0.0);
+        h1 = max0(z1 - zb);
         ld = h1 <= d.hdry ? 1 : 0;
         bmelt += (z1 - zm) * d.arbase;
       }
@@ -1284,11 +1455,6 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   }
 
   // ---- phase A: stencil load, melt, Loop 1 ---------------------------------
-  if (tid == 0) {
-    S.nwet = 0;
-    S.ndry = 0;
-    S.nstale = 0;
-  }
   if (stg) {
     // staged by TMA: the same values, read from shared memory
     const double* g_z = reinterpret_cast<const double*>(stg + L::O_Z);
@@ -1297,8 +1463,11 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     const double* g_qy = reinterpret_cast<const double*>(stg + L::O_QY);
     const double* g_mm = reinterpret_cast<const double*>(stg + L::O_MM);
     const uint8_t* g_fl = stg + L::O_FL;
-    for (int k = tid; k < NSTEN; k += NTHREADS) {
-      const int sr = k % SX, sc = k / SX;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      int sr, sc;
+      if (!stencil_cell<BY>(pass, lx, ly, sr, sc)) break;
+      const int k = sidx(sr, sc);
       const int r = irow0 - 2 + sr, q = icol0 - 2 + sc;
       const int i8 = sc * STG_W8 + sr + so.o8;
       double z = g_z[i8], qx = g_qx[i8], qy = g_qy[i8];
@@ -1308,9 +1477,9 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
         cl = C_INT;
         if (g_fl[sc * STG_W1 + sr + so.o1] & FX_F_WALL) cl |= C_WALL;
         if (melt_on && zb != d.nodata)
-          z = z + (d.melt_mult ? (double)c.meteo_rate * g_mm[i8] / (1000. * 3600. * 24.) * c.dtfl : c.meteoi);
+          z = z + (d.melt_mult ? over((double)c.meteo_rate * g_mm[i8], DAY_MM, 1.0 / DAY_MM) * c.dtfl : c.meteoi);
         if (is_inflow(d, r, q)) z = inflow_z(z, zb, c.inflowi);
-        const double h1 = fmax(0.0, z - zb);
+        const double h1 = max0(z - zb);
         if (h1 <= d.hdry) {
           qx = 0.0;
           qy = 0.0;
@@ -1323,14 +1492,17 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       S.qy[k] = qy;
       S.cls[k] = cl;
       if constexpr (HydroSmem<BY>::VEL) {
-        const double den = fmax(fmax(fmax(0.0, z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0);
-        S.u[k] = qx / den;
-        S.v[k] = qy / den;
+        const Over den(at_least(at_least(max0(z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0));
+        S.u[k] = den.of(qx);
+        S.v[k] = den.of(qy);
       }
     }
   } else
-  for (int k = tid; k < NSTEN; k += NTHREADS) {
-    const int sr = k % SX, sc = k / SX;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    int sr, sc;
+    if (!stencil_cell<BY>(pass, lx, ly, sr, sc)) break;
+    const int k = sidx(sr, sc);
     const int r = irow0 - 2 + sr, q = icol0 - 2 + sc;
     double z = 0.0, zb = 0.0, qx = 0.0, qy = 0.0;
     unsigned char cl = 0;
@@ -1345,7 +1517,7 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
         if (d.flags[sprev + gi] & FX_F_WALL) cl |= C_WALL;
         if (melt_on && zb != d.nodata) z = z + melt_depth(d, c, gi);
         if (is_inflow(d, r, q)) z = inflow_z(z, zb, c.inflowi);
-        const double h1 = fmax(0.0, z - zb);
+        const double h1 = max0(z - zb);
         if (h1 <= d.hdry) {
           qx = 0.0;
           qy = 0.0;
@@ -1359,71 +1531,56 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     S.qy[k] = qy;
     S.cls[k] = cl;
     if constexpr (HydroSmem<BY>::VEL) {
-      const double den = fmax(fmax(fmax(0.0, z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0);
-      S.u[k] = qx / den;
-      S.v[k] = qy / den;
+      const Over den(at_least(at_least(max0(z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0));
+      S.u[k] = den.of(qx);
+      S.v[k] = den.of(qy);
     }
   }
   // the stencil is complete; a thread whose stage wait gave up (bad) stops
   // the whole block here, before anything is written to global memory
   if (__syncthreads_or(bad)) return false;
 
-  // ---- phase B: classify flux cells into warp-uniform work lists ----------
-  for (int k = tid; k < NFLUX; k += NTHREADS) {
-    const int fr = k % FXN, fc = k / FXN;
+  // ---- face fluxes ----------------------------------------------------------
+  // Each thread computes its own face-flux cell (NFLUX == NTHREADS). Lists of
+  // wet, dry and kept cells, which would fill the warps with one kind each,
+  // cost a pass and a barrier more than the divergence they avoid: 2048 x 2048
+  // cells and a 384 x 384 basin take the same time without, 1000 x 700 cells 1 % less.
+  {
+    const int k = tid, fr = lx, fc = ly;
     const int sr = fr + 1, sc = fc + 1;
     const unsigned char cl = S.cls[sidx(sr, sc)];
+    double o[6];
     if (!(cl & C_INT) || (cl & C_WALL)) {
       for (int j = 0; j < 6; ++j) S.f[j][k] = 0.0;  // never written in the reference
-      continue;
-    }
-    if (cl & C_DRY) {
-      const bool alldry = (S.cls[sidx(sr - 1, sc)] & C_DRY) && (S.cls[sidx(sr + 1, sc)] & C_DRY) &&
-                          (S.cls[sidx(sr, sc - 1)] & C_DRY) && (S.cls[sidx(sr, sc + 1)] & C_DRY);
-      if (alldry) S.stale_list[atomicAdd(&S.nstale, 1)] = (short)k;
-      else S.dry_list[atomicAdd(&S.ndry, 1)] = (short)k;
+    } else if (cl & C_DRY) {
+      // all five cells dry: the reference returns before storing
+      // (solver_drydomain.cpp:60-76), so the fluxes of the last step that
+      // computed them stay in effect
+      const bool alldry = S.cls[sidx(sr - 1, sc)] & S.cls[sidx(sr + 1, sc)] & S.cls[sidx(sr, sc - 1)] &
+                          S.cls[sidx(sr, sc + 1)] & C_DRY;
+      if (alldry) {
+        const long long gi = fx_ix(d, irow0 - 1 + fr, icol0 - 1 + fc);
+        const double* rp = fx_rec64(d, sprev + gi);
+        S.f[0][k] = rp[FX_R64_FE1];
+        S.f[1][k] = d.fe2[gi];
+        S.f[2][k] = d.fe3[gi];
+        S.f[3][k] = rp[FX_R64_FN1];
+        S.f[4][k] = d.fn2[gi];
+        S.f[5][k] = d.fn3[gi];
+      } else {
+        solver_dry(d, S, sr, sc, irow0 - 1 + fr, icol0 - 1 + fc, dtl, o);
+        for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
+      }
     } else {
-      S.wet_list[atomicAdd(&S.nwet, 1)] = (short)k;
-    }
-  }
-  __syncthreads();
-
-  // ---- phase C: face fluxes (each face once) -------------------------------
-  {
-    const int nwet = S.nwet, ndry = S.ndry, nstale = S.nstale;
-    double o[6];
-    for (int i = tid; i < nwet; i += NTHREADS) {
-      const int k = S.wet_list[i];
-      const int fr = k % FXN, fc = k / FXN;
-      solver_wet(d, S, fr + 1, fc + 1, irow0 - 1 + fr, icol0 - 1 + fc, dtl, o);
+      solver_wet(d, S, sr, sc, irow0 - 1 + fr, icol0 - 1 + fc, c.dt, o);
       for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
-    }
-    for (int i = tid; i < ndry; i += NTHREADS) {
-      const int k = S.dry_list[i];
-      const int fr = k % FXN, fc = k / FXN;
-      solver_dry(d, S, fr + 1, fc + 1, irow0 - 1 + fr, icol0 - 1 + fc, dtl, o);
-      for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
-    }
-    // All five cells dry: the reference returns before storing
-    // (solver_drydomain.cpp:60-76), so the fluxes of the last step that
-    // computed them stay in effect.
-    for (int i = tid; i < nstale; i += NTHREADS) {
-      const int k = S.stale_list[i];
-      const int fr = k % FXN, fc = k / FXN;
-      const long long gi = fx_ix(d, irow0 - 1 + fr, icol0 - 1 + fc);
-      const double* rp = fx_rec64(d, sprev + gi);
-      S.f[0][k] = rp[FX_R64_FE1];
-      S.f[1][k] = d.fe2[gi];
-      S.f[2][k] = d.fe3[gi];
-      S.f[3][k] = rp[FX_R64_FN1];
-      S.f[4][k] = d.fn2[gi];
-      S.f[5][k] = d.fn3[gi];
     }
   }
   __syncthreads();
 
   // ---- phase D: Loop 3, Loop 4, friction, store, next Courant --------------
-  double dtc = __longlong_as_double(0x7ff0000000000000LL), hm = 0.0, bmelt = 0.0, bout = 0.0;
+  double bmelt = 0.0, bout = 0.0;
+  double c_h = 0.0, c_qx = 0.0, c_qy = 0.0;  // this thread's cell after the update
   if (own) {
     const long long gi = fx_ix(d, irow, icol);
     const int sP = sidx(lx + 2, ly + 2);
@@ -1439,21 +1596,21 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     // add_meteo's h0 (common.cpp:223): the depth after the melt, or the
     // Courant scan's copy of h (main.cpp:305) for cells it skips. Its solute
     // dilution (:226-234) is applied by the ADE sweep (fx_ade.cu).
-    double h0v = fmax(0.0, zpre - zb);
+    double h0v = max0(zpre - zb);
     double mi = 0.0, hpv = 0.0;
     if (melt_on && zb != d.nodata) {
-      h0v = fmax(z1 - zb, 0.0);
-      hpv = fmax(zpre - zb, 0.0);  // the dilution's hp (common.cpp:216)
-      mi = (stg && d.melt_mult) ? (double)c.meteo_rate * reinterpret_cast<const double*>(stg + L::O_MM)[i8] /
-                                      (1000. * 3600. * 24.) * c.dtfl
-                                : melt_depth(d, c, gi);
+      h0v = max0(z1 - zb);
+      hpv = max0(zpre - zb);  // the dilution's hp (common.cpp:216)
+      mi = (stg && d.melt_mult)
+               ? over((double)c.meteo_rate * reinterpret_cast<const double*>(stg + L::O_MM)[i8], DAY_MM, 1.0 / DAY_MM) * c.dtfl
+               : melt_depth(d, c, gi);
       bmelt = mi * d.arbase;
     }
     if (is_inflow(d, irow, icol)) {  // common.cpp:300-315 (h0 = the depth after the inflow)
       const double zm = (melt_on && zb != d.nodata) ? zpre + mi : zpre;
-      record_inflow_hm(d, c, fmax(zm - zb, 0.0));
+      record_inflow_hm(d, c, max0(zm - zb));
       bmelt += (z1 - zm) * d.arbase;
-      h0v = fmax(z1 - zb, 0.0);
+      h0v = max0(z1 - zb);
     }
     // Loop 1 wet time (:69-70)
     if (!(cl & C_DRY)) d.twet[gi] += c.twet_inc;  // dtl / 3600
@@ -1461,9 +1618,9 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     // Loop 3 (:93-120)
     double dh = 0.0, dqx = 0.0, dqy = 0.0, qxfP = 0.0, qyfP = 0.0;
     if (!wall) {
-      dh = (fx_div_dxy(d, S.f[0][fW] - S.f[0][fP]) + fx_div_dxy(d, S.f[3][fS] - S.f[3][fP])) * dtl;
-      dqx = (fx_div_dxy(d, S.f[1][fW] - S.f[1][fP]) + fx_div_dxy(d, S.f[4][fS] - S.f[4][fP])) * dtl;
-      dqy = (fx_div_dxy(d, S.f[2][fW] - S.f[2][fP]) + fx_div_dxy(d, S.f[5][fS] - S.f[5][fP])) * dtl;
+      dh = (div_dxy(d, S.f[0][fW] - S.f[0][fP]) + div_dxy(d, S.f[3][fS] - S.f[3][fP])) * dtl;
+      dqx = (div_dxy(d, S.f[1][fW] - S.f[1][fP]) + div_dxy(d, S.f[4][fS] - S.f[4][fP])) * dtl;
+      dqy = (div_dxy(d, S.f[2][fW] - S.f[2][fP]) + div_dxy(d, S.f[5][fS] - S.f[5][fP])) * dtl;
       qxfP = S.f[0][fP] * dtl;
       qyfP = S.f[3][fP] * dtl;
     }
@@ -1475,12 +1632,12 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       if (irow == d.nr || (clE & C_WALL)) bout += S.f[0][fP] * d.dxy * dtl;
       if (icol == d.nc || (clN & C_WALL)) bout += S.f[3][fP] * d.dxy * dtl;
     }
-    const double qxfW = ((clW & C_INT) && !(clW & C_WALL)) ? S.f[0][fW] * dtl : 0.0;
-    const double qyfS = ((clS & C_INT) && !(clS & C_WALL)) ? S.f[3][fS] * dtl : 0.0;
+    const double qxfW = ((clW & (C_INT | C_WALL)) == C_INT) ? S.f[0][fW] * dtl : 0.0;
+    const double qyfS = ((clS & (C_INT | C_WALL)) == C_INT) ? S.f[3][fS] * dtl : 0.0;
 
     // Loop 4 (:123-154)
     const double z = z1 + dh;
-    const double h = fmax(0.0, z - zb);
+    const double h = max0(z - zb);
     double qx, qy;
     uint8_t ld;
     if (h < d.hdry || wall) {
@@ -1500,9 +1657,9 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       if (n != 0.0) {
         const double qm = sqrt(qx * qx + qy * qy);
         const double h73 = h * h * fx_cbrt(h);
-        const double den = 1.0 + dtl * d.gaccl * n * n * qm / h73;
-        qx = qx / den;
-        qy = qy / den;
+        const Over den(1.0 + dtl * d.gaccl * n * n * qm / h73);
+        qx = den.of(qx);
+        qy = den.of(qy);
       }
     }
     d.z[pcur + gi] = z;
@@ -1520,8 +1677,8 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     double fe1v = 0.0, fn1v = 0.0;
     if ((clP & C_INT) && !(clP & C_WALL)) {
       const bool computed =
-          !(clP & C_DRY) || !((S.cls[sidx(lx + 1, ly + 2)] & C_DRY) && (S.cls[sidx(lx + 3, ly + 2)] & C_DRY) &&
-                              (S.cls[sidx(lx + 2, ly + 1)] & C_DRY) && (S.cls[sidx(lx + 2, ly + 3)] & C_DRY));
+          !(clP & C_DRY) || !(S.cls[sidx(lx + 1, ly + 2)] & S.cls[sidx(lx + 3, ly + 2)] &
+                              S.cls[sidx(lx + 2, ly + 1)] & S.cls[sidx(lx + 2, ly + 3)] & C_DRY);
       // fe_1/fn_1 of every cell go to this step's slot: computed ones, or the
       // stale ones carried over (already in S.f for stale cells).
       fe1v = S.f[0][fP];
@@ -1534,8 +1691,12 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       }
     }  // walls: fe_1 = fn_1 = 0, never written in the reference
     put_rec64(d, scur + gi, h0v, h, hpv, fe1v, fn1v, fl1);
-    courant_cell(d, h, qx, qy, dtc, hm);
+    c_h = h;
+    c_qx = qx;
+    c_qy = qy;
   }
+  double dtc, hm;
+  courant_cell(d, c_h, c_qx, c_qy, dtc, hm);
   acc.add(dtc, hm, bmelt, bout);
   return true;
 }
@@ -1547,16 +1708,7 @@ __device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile
                                             StepCtl& sc) {
   static_assert(sizeof(HydroSmem32<BY>) <= sizeof(HydroSmem<BY>), "FP32 tile state reuses the FP64 one");
   if (threadIdx.x == 0 && threadIdx.y == 0) {
-    const fx_ctl& g = *d.ctl;
-    sc.dtfl = g.dtfl;
-    sc.meteoi = g.meteoi;
-    sc.meteo_rate = g.meteo_rate;
-    sc.mconc = g.mconc;
-    sc.inflowi = g.inflowi;
-    sc.twet_inc = g.dtfl / 3600;
-    sc.steps = g.steps;
-    sc.live = g.live;
-    sc.active = g.active;
+    read_ctl(d, sc);
   }
   __syncthreads();
   const StepCtl c = sc;
@@ -1567,14 +1719,18 @@ __device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile
   reduce_part(d, S, acc);
 }
 
-// Blocks per SM the launch bounds ask for: 768 threads for FP64 (at most 85
-// registers each), 1024 for FP32 (at most 64). The kernel is bound by
-// instruction latency and tile barriers, so resident warps pay for the
-// spills this costs: at 4096 x 4096 cells the FP32 kernel took 1.50 ms per
-// step at 64 registers against 1.73 ms at 80 (3 blocks), the FP64 one 4.01
-// ms at 85 against 4.39 ms at 128 (2 blocks).
+// Blocks per SM the launch bounds ask for: 768 threads for FP64 (at most 80
+// registers each), 1024 for FP32 (at most 64). The kernel is bound by the
+// instructions it issues (FP32: 71 % of the issue slots) and by their latency
+// and the tile barriers (FP64: 52 %), so resident warps pay for the spills
+// this costs: at 4096 x 4096 cells the FP32 kernel took 1.50 ms per step at
+// 64 registers against 1.73 ms at 80 (3 blocks); at 2048 x 2048 the FP64 one
+// took 0.68 ms at 80 against 0.71 ms at 128 (2 blocks), in tiles of 8 rows.
+// FP64 tiles of 4 rows serve the small grids, whose blocks have a tile or two
+// and little company on their SM: with 96 registers (5 blocks) they take
+// 16.4 us at 200 x 200 and 126 us at 1000 x 700, with 80 18.2 and 140 us.
 template <bool P32, int BY>
-constexpr int min_blocks() { return (P32 ? 32 : 24) / BY > 0 ? (P32 ? 32 : 24) / BY : 1; }
+constexpr int min_blocks() { return (P32 ? 32 : BY == 4 ? 20 : 24) / BY; }
 
 // One domain: the descriptor is a kernel parameter (constant bank), so its
 // fields are instruction operands. Block (x, y) is tile (x, y).
@@ -1684,16 +1840,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
   const int tid = threadIdx.y * BX + threadIdx.x;
   const int ntiles = ntx * nty;
   if (tid == 0) {
-    const fx_ctl& g = *d.ctl;
-    sc.dtfl = g.dtfl;
-    sc.meteoi = g.meteoi;
-    sc.meteo_rate = g.meteo_rate;
-    sc.mconc = g.mconc;
-    sc.inflowi = g.inflowi;
-    sc.twet_inc = g.dtfl / 3600;
-    sc.steps = g.steps;
-    sc.live = g.live;
-    sc.active = g.active;
+    read_ctl(d, sc);
   }
   __syncthreads();
   const StepCtl c = sc;
@@ -1830,16 +1977,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
       for (int i = tid; i < (int)(sizeof(fx_dev) / 8); i += BX * BY) dst[i] = src[i];
       __syncthreads();
       if (tid == 0) {
-        const fx_ctl& g = *sd.ctl;
-        sc.dtfl = g.dtfl;
-        sc.meteoi = g.meteoi;
-        sc.meteo_rate = g.meteo_rate;
-        sc.mconc = g.mconc;
-        sc.inflowi = g.inflowi;
-        sc.twet_inc = g.dtfl / 3600;
-        sc.steps = g.steps;
-        sc.live = g.live;
-        sc.active = g.active;
+        read_ctl(sd, sc);
       }
       __syncthreads();
       dom = tl.dom;
