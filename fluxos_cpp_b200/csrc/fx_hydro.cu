@@ -20,6 +20,7 @@
 // reference bit for bit except where noted at fx_pow15.
 #include <cuda_runtime.h>
 
+#include <type_traits>
 #include <vector>
 
 #include "fx_common.cuh"
@@ -50,18 +51,20 @@ constexpr unsigned char C_DRY = 1;   // Loop-1 ldry == 1 (interior cells only)
 constexpr unsigned char C_WALL = 2;  // innerNeumannBCWeir == 1
 constexpr unsigned char C_INT = 4;   // interior cell (1..NROWS, 1..NCOLS)
 
-template <int BY>
-struct HydroSmem {
+template <int BY, bool STAGED>
+struct HydroSmem64 {
   static constexpr int NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX, NW = Tile<BY>::NTHREADS / 32;
   double budget[2 * NW];
-  double z[NSTEN], zb[NSTEN], qx[NSTEN], qy[NSTEN];
+  double z[NSTEN], qx[NSTEN], qy[NSTEN];
+  double mi[STAGED ? NSTEN : 1];  // the step's melt depth, of the cells that take it
+  double zb[STAGED ? 1 : NSTEN];  // a staged tile reads the bed where TMA left it
   // cell velocities q / max(h, hdry, ks) of the stencil, formed once per
   // cell for the wet solver's shear terms (the same expression and operands
   // the solver divides for each face, so the same values); kept for tiles
   // up to 8 rows, the largest tile's state stays within 48 KB
   static constexpr bool VEL = BY <= 8;
   double u[VEL ? NSTEN : 1], v[VEL ? NSTEN : 1];
-  double f[6][NFLUX];
+  double f[3][NFLUX];  // north face fluxes
   unsigned char cls[NSTEN];
   double red_dt[NW], red_h[NW];
 };
@@ -182,17 +185,23 @@ __device__ __forceinline__ bool stencil_cell(int pass, int lx, int ly, int& sr, 
 }
 
 __device__ __forceinline__ int sidx(int sr, int sc) { return sc * SX + sr; }
+// The bed of the tile's stencil: columns LD doubles apart.
+template <int LD>
+struct Bed {
+  const double* p;
+  __device__ __forceinline__ double operator()(int sr, int sc) const { return p[sc * LD + sr]; }
+};
 
 // solver_wetdomain.cpp:27-342 for the flux cell at stencil (sr, sc).
-template <class SM>
-__device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
+template <class SM, class BED>
+__device__ void solver_wet(const fx_dev& d, const SM& S, const BED& bed, int sr, int sc, int irow, int icol,
                            Over dt, double out[6]) {
   const double hdryl = d.hdry, gaccl = d.gaccl;
   const int P = sidx(sr, sc), W = sidx(sr - 1, sc), E = sidx(sr + 1, sc);
   const int Sx = sidx(sr, sc - 1), N = sidx(sr, sc + 1);
   const int ES = sidx(sr + 1, sc - 1), EN = sidx(sr + 1, sc + 1), WN = sidx(sr - 1, sc + 1);
   auto ksat = [&](int k) { return (S.cls[k] & C_INT) ? d.ks : 0.0; };
-  auto hat = [&](int k) { return max0(S.z[k] - S.zb[k]); };
+  auto hat = [&](int r, int q) { return max0(S.z[sidx(r, q)] - bed(r, q)); };
   const double kspl = ksat(P);
   const double nueml = d.nueml, cvdefl = d.cvdefl;
   const unsigned dx = d.dxy_u, dy = d.dxy_u;
@@ -202,7 +211,8 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
   const bool lde_dry = S.cls[E] & C_DRY;
   const bool ldn_dry = S.cls[N] & C_DRY;
 
-  const double zbw = S.zb[W], zbp = S.zb[P], zbe = S.zb[E], zbs = S.zb[Sx], zbn = S.zb[N];
+  const double zbw = bed(sr - 1, sc), zbp = bed(sr, sc), zbe = bed(sr + 1, sc);
+  const double zbs = bed(sr, sc - 1), zbn = bed(sr, sc + 1);
   const double zw = S.z[W], zp = S.z[P], ze = S.z[E], zs = S.z[Sx], zn = S.z[N];
   double qp = S.qx[P], qe = S.qx[E], qn = S.qx[N];
   double rw = S.qy[W], rp = S.qy[P], re = S.qy[E], rn = S.qy[N];
@@ -312,12 +322,12 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
     vp = hp_.of(rp);
     un = qn / fmax(fmax(hn, hdryl), ksat(N));
     us0 = S.qx[Sx] / fmax(fmax(hs, hdryl), ksat(Sx));
-    use0 = S.qx[ES] / fmax(fmax(hat(ES), hdryl), ksat(ES));
-    une = S.qx[EN] / fmax(fmax(hat(EN), hdryl), ksat(EN));
+    use0 = S.qx[ES] / fmax(fmax(hat(sr + 1, sc - 1), hdryl), ksat(ES));
+    une = S.qx[EN] / fmax(fmax(hat(sr + 1, sc + 1), hdryl), ksat(EN));
     ve = re / fmax(fmax(he, hdryl), ksat(E));
     vw = rw / fmax(fmax(hw, hdryl), ksat(W));
-    vwn = S.qy[WN] / fmax(fmax(hat(WN), hdryl), ksat(WN));
-    ven = S.qy[EN] / fmax(fmax(hat(EN), hdryl), ksat(EN));
+    vwn = S.qy[WN] / fmax(fmax(hat(sr - 1, sc + 1), hdryl), ksat(WN));
+    ven = S.qy[EN] / fmax(fmax(hat(sr + 1, sc + 1), hdryl), ksat(EN));
   }
 
   const double txye = hne * (div_dxy(d, ve - vp) + div_dxy(d, .25 * (un + une - us0 - use0)));
@@ -425,14 +435,14 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, int sr, int sc, int iro
 }
 
 // solver_drydomain.cpp:78-194 (the cell is dry and has a wet neighbour).
-template <class SM>
-__device__ void solver_dry(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
+template <class SM, class BED>
+__device__ void solver_dry(const fx_dev& d, const SM& S, const BED& bed, int sr, int sc, int irow, int icol,
                            double dtl, double out[6]) {
   const int P = sidx(sr, sc), E = sidx(sr + 1, sc), N = sidx(sr, sc + 1);
   const double gaccl = d.gaccl;
   double volrat = d.volrat_mode == 0 ? __longlong_as_double(0x7ff0000000000000LL) : 0.0;
   const bool lde_dry = S.cls[E] & C_DRY, ldn_dry = S.cls[N] & C_DRY;
-  const double zbp = S.zb[P], zbe = S.zb[E], zbn = S.zb[N];
+  const double zbp = bed(sr, sc), zbe = bed(sr + 1, sc), zbn = bed(sr, sc + 1);
   const double zp = S.z[P], ze = S.z[E], zn = S.z[N];
   const double hp = fmax(0.0, zp - zp);  // :85 reads z - z
   const double he = fmax(0.0, ze - zbe);
@@ -706,21 +716,24 @@ __device__ __forceinline__ void record_inflow_hm(const fx_dev& d, const StepCtl&
 // the signs of near-zero surface differences are decided in FP64 on the
 // compensated depth; the Courant candidates and the water budget are FP64.
 
-template <int BY>
+template <int BY, bool STAGED>
 struct HydroSmem32 {
   static constexpr int NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX, NW = Tile<BY>::NTHREADS / 32;
   double budget[2 * NW];
   double red_dt[NW], red_h[NW];
-  double zb[NSTEN];
+  double zb[STAGED ? 1 : NSTEN];
   float eta[NSTEN], eta_lo[NSTEN], qx[NSTEN], qy[NSTEN];
   // cell velocities q / max(h, hdry, ks) of the stencil, formed once per
   // cell for the wet solver's shear terms (each face reads eight of them)
   static constexpr bool VEL = true;
   float u[NSTEN], v[NSTEN];
   float mi[NSTEN];  // the step's melt depth, of the cells that take it
-  float f[6][NFLUX];
+  float f[3][NFLUX];  // north face fluxes
   unsigned char cls[NSTEN];
 };
+
+template <bool P32, int BY, bool STAGED>
+using HydroSmem = std::conditional_t<P32, HydroSmem32<BY, STAGED>, HydroSmem64<BY, STAGED>>;
 
 // FP32 arithmetic divides and takes square roots by the approximate hardware
 // reciprocal and square root (PTX rcp.approx / sqrt.approx) refined by one
@@ -844,8 +857,8 @@ __device__ __forceinline__ bool dd_lt_hdry(const fx_dev& d, float eta, float lo)
   return fx_dd_val(eta, lo) < d.hdry;
 }
 
-template <class SM>
-__device__ void solver_wet32(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
+template <class SM, class BED>
+__device__ void solver_wet32(const fx_dev& d, const SM& S, const BED& bed, int sr, int sc, int irow, int icol,
                              float dtl, float out[6]) {
   const double hdry = d.hdry;
   const float hdryl = d.f.hdry, gaccl = d.f.gaccl, hdry_lo = d.f.hdry_lo, hdry_hi = d.f.hdry_hi;
@@ -860,7 +873,7 @@ __device__ void solver_wet32(const fx_dev& d, const SM& S, int sr, int sc, int i
   float volrat = d.volrat_mode == 0 ? __int_as_float(0x7f800000) : 0.0f;
   const bool ldp_dry = S.cls[P] & C_DRY, lde_dry = S.cls[E] & C_DRY, ldn_dry = S.cls[N] & C_DRY;
   // bed differences: exact in FP64 for the branch tests, rounded for the flux arithmetic
-  const double sx_d = S.zb[E] - S.zb[P], sy_d = S.zb[N] - S.zb[P];
+  const double sx_d = bed(sr + 1, sc) - bed(sr, sc), sy_d = bed(sr, sc + 1) - bed(sr, sc);
   const float etap = S.eta[P], sxp = (float)sx_d, syp = (float)sy_d;
   // compensated depths for the branch tests (FP64, as the FP64 path decides
   // them), formed where a test needs them
@@ -1009,14 +1022,14 @@ __device__ void solver_wet32(const fx_dev& d, const SM& S, int sr, int sc, int i
   out[5] = fn3;
 }
 
-template <class SM>
-__device__ void solver_dry32(const fx_dev& d, const SM& S, int sr, int sc, int irow, int icol,
+template <class SM, class BED>
+__device__ void solver_dry32(const fx_dev& d, const SM& S, const BED& bed, int sr, int sc, int irow, int icol,
                              float dtl, float out[6]) {
   const int P = sidx(sr, sc), E = sidx(sr + 1, sc), N = sidx(sr, sc + 1);
   const float gaccl = d.f.gaccl;
   float volrat = d.volrat_mode == 0 ? __int_as_float(0x7f800000) : 0.0f;
   const bool lde_dry = S.cls[E] & C_DRY, ldn_dry = S.cls[N] & C_DRY;
-  const double sx_d = S.zb[E] - S.zb[P], sy_d = S.zb[N] - S.zb[P];
+  const double sx_d = bed(sr + 1, sc) - bed(sr, sc), sy_d = bed(sr, sc + 1) - bed(sr, sc);
   const float etap = S.eta[P], etae = S.eta[E], etan = S.eta[N], sxp = (float)sx_d, syp = (float)sy_d;
   const double dP = fx_dd_val(etap, S.eta_lo[P]), dE = fx_dd_val(etae, S.eta_lo[E]);
   const double dN = fx_dd_val(etan, S.eta_lo[N]);
@@ -1092,10 +1105,63 @@ __device__ __forceinline__ void put_rec32(const fx_dev& d, long long o, float h0
   r[1] = make_float4(fe1, fn1, __uint_as_float((unsigned)fl), 0.0f);
 }
 
+// A step without solver (no wet cell): the Courant scan and add_meteo only
+// (main.cpp:300-370, the solver block at :385 is skipped).
 template <int BY>
+__device__ __forceinline__ void idle_tile32(const fx_dev& d, const StepCtl& c, const fx_tile& tile, TilePart& acc) {
+  const int irow = 1 + tile.bx * TX + threadIdx.x, icol = 1 + tile.by * Tile<BY>::TY + threadIdx.y;
+  const bool own = threadIdx.x < TX && threadIdx.y < Tile<BY>::TY && irow <= d.nr && icol <= d.nc;
+  const bool melt_on = d.has_meteo != 0;
+  const long long sprev = c.sprev, scur = c.scur, pprev = c.pprev, pcur = c.pcur;
+  double dtc = __longlong_as_double(0x7ff0000000000000LL), hm = 0.0, bmelt = 0.0;
+  if (own) {
+    const long long gi = fx_ix(d, irow, icol);
+    const float etapre = d.eta[pprev + gi];
+    float eta1 = etapre, lo1 = d.eta_lo[pprev + gi];
+    const uint8_t fl = d.flags[sprev + gi];
+    const float hpre = fmaxf(0.0f, etapre);
+    uint8_t ld = fx_dd_val(etapre, lo1) > d.hdry ? 0 : 1;
+    float h1 = hpre;
+    double depth = fx_dd_val(etapre, lo1);
+    float mir = 0.0f;  // the record's melt depth
+    if (melt_on && !(fl & FX_F_NODATA)) {
+      const float mi = melt32(d, c, d.melt_mult_f ? d.melt_mult_f[gi] : 1.0f);
+      mir = mi;
+      bmelt = (double)mi * d.arbase;
+      fx_dd_add(eta1, lo1, mi);
+      h1 = fmaxf(eta1, 0.0f);
+      depth = fx_dd_val(eta1, lo1);
+      if (depth <= d.hdry) ld = 0;
+    }
+    if (is_inflow(d, irow, icol)) {  // common.cpp:300-315
+      const double dm = fx_dd_val(eta1, lo1);
+      record_inflow_hm(d, c, fmax(dm, 0.0));
+      inflow_eta(eta1, lo1, c.inflowi);
+      depth = fx_dd_val(eta1, lo1);
+      bmelt += (depth - dm) * d.arbase;
+      h1 = fmaxf(eta1, 0.0f);
+      ld = depth <= d.hdry ? 1 : 0;
+    }
+    const float qx = d.qx_f[pprev + gi], qy = d.qy_f[pprev + gi];
+    d.eta[pcur + gi] = eta1;
+    d.eta_lo[pcur + gi] = lo1;
+    d.qx_f[pcur + gi] = qx;
+    d.qy_f[pcur + gi] = qy;
+    const uint8_t fl1 = (fl & (FX_F_WALL | FX_F_NODATA)) | ((fl & FX_F_LDRY) ? FX_F_LDRY_PREV : 0) | ld;
+    d.flags[scur + gi] = fl1;
+    // fluxes are unchanged by a step without solver
+    const float* rp = fx_rec(d, sprev + gi);
+    const bool melted = melt_on && !(fl & FX_F_NODATA);
+    put_rec32(d, scur + gi, h1, h1, melted ? hpre : 0.0f, mir,
+              rp[FX_R_FE1], rp[FX_R_FN1], fl1);
+    courant_cell32(d, fmax(0.0, depth), qx, qy, dtc, hm);
+  }
+  acc.add(dtc, hm, bmelt, 0.0);
+}
+
+template <int BY, bool STAGED>
 __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, const fx_tile& tile,
-                                             HydroSmem32<BY>& S, TilePart& acc, const unsigned char* stg = nullptr,
-                                             int bad = 0) {
+                                             HydroSmem32<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad) {
   using L = StageLayout<true, BY>;
   const StageOff so = stage_off(tile.bx);
   constexpr int TY = Tile<BY>::TY, NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX;
@@ -1103,65 +1169,24 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
   const int lx = threadIdx.x, ly = threadIdx.y;
   const int tid = ly * BX + lx;
   const int irow0 = 1 + tile.bx * TX, icol0 = 1 + tile.by * TY;
-  const int irow = irow0 + lx, icol = icol0 + ly;
-  const bool own = lx < TX && ly < TY && irow <= d.nr && icol <= d.nc;
+  // The thread's face-flux cell and, but for the west row and south column of
+  // the tile, the cell it owns.
+  const int irow = irow0 - 1 + lx, icol = icol0 - 1 + ly;
+  const bool own = lx > 0 && ly > 0 && irow <= d.nr && icol <= d.nc;
   const float dtl = c.dtf;
   const bool melt_on = d.has_meteo != 0;
   const long long sprev = c.sprev, scur = c.scur, pprev = c.pprev, pcur = c.pcur;
-  double dtc = __longlong_as_double(0x7ff0000000000000LL), hm = 0.0, bmelt = 0.0, bout = 0.0;
+  double bmelt = 0.0, bout = 0.0;
 
-  if (!c.active) {
-    if (own) {
-      const long long gi = fx_ix(d, irow, icol);
-      const float etapre = d.eta[pprev + gi];
-      float eta1 = etapre, lo1 = d.eta_lo[pprev + gi];
-      const uint8_t fl = d.flags[sprev + gi];
-      const float hpre = fmaxf(0.0f, etapre);
-      uint8_t ld = fx_dd_val(etapre, lo1) > d.hdry ? 0 : 1;
-      float h1 = hpre;
-      double depth = fx_dd_val(etapre, lo1);
-      float mir = 0.0f;  // the record's melt depth
-      if (melt_on && !(fl & FX_F_NODATA)) {
-        const float mi = melt32(d, c, d.melt_mult_f ? d.melt_mult_f[gi] : 1.0f);
-        mir = mi;
-        bmelt = (double)mi * d.arbase;
-        fx_dd_add(eta1, lo1, mi);
-        h1 = fmaxf(eta1, 0.0f);
-        depth = fx_dd_val(eta1, lo1);
-        if (depth <= d.hdry) ld = 0;
-      }
-      if (is_inflow(d, irow, icol)) {  // common.cpp:300-315
-        const double dm = fx_dd_val(eta1, lo1);
-        record_inflow_hm(d, c, fmax(dm, 0.0));
-        inflow_eta(eta1, lo1, c.inflowi);
-        depth = fx_dd_val(eta1, lo1);
-        bmelt += (depth - dm) * d.arbase;
-        h1 = fmaxf(eta1, 0.0f);
-        ld = depth <= d.hdry ? 1 : 0;
-      }
-      const float qx = d.qx_f[pprev + gi], qy = d.qy_f[pprev + gi];
-      d.eta[pcur + gi] = eta1;
-      d.eta_lo[pcur + gi] = lo1;
-      d.qx_f[pcur + gi] = qx;
-      d.qy_f[pcur + gi] = qy;
-      const uint8_t fl1 = (fl & (FX_F_WALL | FX_F_NODATA)) | ((fl & FX_F_LDRY) ? FX_F_LDRY_PREV : 0) | ld;
-      d.flags[scur + gi] = fl1;
-      // fluxes are unchanged by a step without solver
-      const float* rp = fx_rec(d, sprev + gi);
-      const bool melted = melt_on && !(fl & FX_F_NODATA);
-      put_rec32(d, scur + gi, h1, h1, melted ? hpre : 0.0f, mir,
-                rp[FX_R_FE1], rp[FX_R_FN1], fl1);
-      courant_cell32(d, fmax(0.0, depth), qx, qy, dtc, hm);
-    }
-    acc.add(dtc, hm, bmelt, 0.0);
-    return true;
-  }
 
-  if (stg) {
+  const auto bed = [&] {
+    if constexpr (STAGED) return Bed<STG_W8>{reinterpret_cast<const double*>(stg + L::O_ZB) + so.o8};
+    else return Bed<SX>{S.zb};
+  }();
+  if constexpr (STAGED) {
     // staged by TMA: the same values, read from shared memory
     const float* g_eta = reinterpret_cast<const float*>(stg + L::O_Z);
     const float* g_lo = reinterpret_cast<const float*>(stg + L::O_LO);
-    const double* g_zb = reinterpret_cast<const double*>(stg + L::O_ZB);
     const float* g_qx = reinterpret_cast<const float*>(stg + L::O_QX);
     const float* g_qy = reinterpret_cast<const float*>(stg + L::O_QY);
     const float* g_mm = reinterpret_cast<const float*>(stg + L::O_MM);
@@ -1174,7 +1199,6 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       const int r = irow0 - 2 + sr, q = icol0 - 2 + scc;
       const int i4 = scc * STG_W4 + sr + so.o4;
       float eta = g_eta[i4], lo = g_lo[i4], qx = g_qx[i4], qy = g_qy[i4];
-      const double zb = g_zb[scc * STG_W8 + sr + so.o8];
       unsigned char cl = 0;
       if (r >= 1 && r <= d.nr && q >= 1 && q <= d.nc) {
         cl = C_INT;
@@ -1194,7 +1218,6 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       }
       S.eta[k] = eta;
       S.eta_lo[k] = lo;
-      S.zb[k] = zb;
       S.qx[k] = qx;
       S.qy[k] = qy;
       S.cls[k] = cl;
@@ -1204,100 +1227,102 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
         S.v[k] = fdiv(qy, den);
       }
     }
-  } else
+  } else {
 #pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-    int sr, scc;
-    if (!stencil_cell<BY>(pass, lx, ly, sr, scc)) break;
-    const int k = sidx(sr, scc);
-    const int r = irow0 - 2 + sr, q = icol0 - 2 + scc;
-    float eta = 0.f, lo = 0.f, qx = 0.f, qy = 0.f;
-    double zb = 0.0;
-    unsigned char cl = 0;
-    if (r >= 0 && r <= d.nr + 1 && q >= 0 && q <= d.nc + 1) {
-      const long long gi = fx_ix(d, r, q);
-      eta = d.eta[pprev + gi];
-      lo = d.eta_lo[pprev + gi];
-      zb = d.zb[gi];
-      qx = d.qx_f[pprev + gi];
-      qy = d.qy_f[pprev + gi];
-      if (r >= 1 && r <= d.nr && q >= 1 && q <= d.nc) {
-        cl = C_INT;
-        const uint8_t fl = d.flags[sprev + gi];
-        if (fl & FX_F_WALL) cl |= C_WALL;
-        if (melt_on && !(fl & FX_F_NODATA)) {
-          const float mi = melt32(d, c, d.melt_mult_f ? d.melt_mult_f[gi] : 1.0f);
-          S.mi[k] = mi;
-          fx_dd_add(eta, lo, mi);
-        }
-        if (is_inflow(d, r, q)) inflow_eta(eta, lo, c.inflowi);
-        if (dd_le_hdry(d, eta, lo)) {
-          qx = 0.f;
-          qy = 0.f;
-          cl |= C_DRY;
+    for (int pass = 0; pass < 2; ++pass) {
+      int sr, scc;
+      if (!stencil_cell<BY>(pass, lx, ly, sr, scc)) break;
+      const int k = sidx(sr, scc);
+      const int r = irow0 - 2 + sr, q = icol0 - 2 + scc;
+      float eta = 0.f, lo = 0.f, qx = 0.f, qy = 0.f;
+      double zb = 0.0;
+      unsigned char cl = 0;
+      if (r >= 0 && r <= d.nr + 1 && q >= 0 && q <= d.nc + 1) {
+        const long long gi = fx_ix(d, r, q);
+        eta = d.eta[pprev + gi];
+        lo = d.eta_lo[pprev + gi];
+        zb = d.zb[gi];
+        qx = d.qx_f[pprev + gi];
+        qy = d.qy_f[pprev + gi];
+        if (r >= 1 && r <= d.nr && q >= 1 && q <= d.nc) {
+          cl = C_INT;
+          const uint8_t fl = d.flags[sprev + gi];
+          if (fl & FX_F_WALL) cl |= C_WALL;
+          if (melt_on && !(fl & FX_F_NODATA)) {
+            const float mi = melt32(d, c, d.melt_mult_f ? d.melt_mult_f[gi] : 1.0f);
+            S.mi[k] = mi;
+            fx_dd_add(eta, lo, mi);
+          }
+          if (is_inflow(d, r, q)) inflow_eta(eta, lo, c.inflowi);
+          if (dd_le_hdry(d, eta, lo)) {
+            qx = 0.f;
+            qy = 0.f;
+            cl |= C_DRY;
+          }
         }
       }
+      S.eta[k] = eta;
+      S.eta_lo[k] = lo;
+      S.zb[k] = zb;
+      S.qx[k] = qx;
+      S.qy[k] = qy;
+      S.cls[k] = cl;
+        {
+          const float den = fmaxf(fmaxf(fmaxf(0.0f, eta), d.f.hdry), (cl & C_INT) ? d.f.ks : 0.0f);
+          S.u[k] = fdiv(qx, den);
+          S.v[k] = fdiv(qy, den);
+        }
     }
-    S.eta[k] = eta;
-    S.eta_lo[k] = lo;
-    S.zb[k] = zb;
-    S.qx[k] = qx;
-    S.qy[k] = qy;
-    S.cls[k] = cl;
-      {
-        const float den = fmaxf(fmaxf(fmaxf(0.0f, eta), d.f.hdry), (cl & C_INT) ? d.f.ks : 0.0f);
-        S.u[k] = fdiv(qx, den);
-        S.v[k] = fdiv(qy, den);
-      }
   }
   // the stencil is complete; a thread whose stage wait gave up (bad) stops
   // the whole block here, before anything is written to global memory
   if (__syncthreads_or(bad)) return false;
-  {
-    // Each thread computes its own face-flux cell (NFLUX == NTHREADS), wet,
-    // dry or kept: gathering each kind's cells in lists cost more than the
-    // divergence it avoids (4096^2 wet start 1.4 % and the 64-scenario batch
-    // 6 % faster without).
-    const int k = tid, fr = lx, fc = ly;
-    const int sr = fr + 1, scc = fc + 1;
-    const unsigned char cl = S.cls[sidx(sr, scc)];
-    float o[6];
-    if (!(cl & C_INT) || (cl & C_WALL)) {
-      for (int j = 0; j < 6; ++j) S.f[j][k] = 0.0f;
-    } else if (cl & C_DRY) {
-      const bool alldry = S.cls[sidx(sr - 1, scc)] & S.cls[sidx(sr + 1, scc)] & S.cls[sidx(sr, scc - 1)] &
-                          S.cls[sidx(sr, scc + 1)] & C_DRY;
-      if (alldry) {  // all five cells dry: the last computed fluxes stay (solver_drydomain.cpp:60-76)
-        const long long gi = fx_ix(d, irow0 - 1 + fr, icol0 - 1 + fc);
-        const float* rp = fx_rec(d, sprev + gi);
-        S.f[0][k] = rp[FX_R_FE1];
-        S.f[1][k] = d.fe2_f[gi];
-        S.f[2][k] = d.fe3_f[gi];
-        S.f[3][k] = rp[FX_R_FN1];
-        S.f[4][k] = d.fn2_f[gi];
-        S.f[5][k] = d.fn3_f[gi];
-      } else {
-        solver_dry32(d, S, sr, scc, irow0 - 1 + fr, icol0 - 1 + fc, dtl, o);
-        for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
-      }
+  // Each thread computes its own face-flux cell (NFLUX == NTHREADS), wet, dry
+  // or kept: gathering each kind's cells in lists cost more than the
+  // divergence it avoids (4096^2 wet start 1.4 % and the 64-scenario batch 6 %
+  // faster without).
+  // Its six fluxes stay in registers for the update of the cell itself; the
+  // east faces' go to the neighbour's lane by shuffle, the north faces' to the
+  // next column's warp through shared memory.
+  const int sr = lx + 1, sc = ly + 1, sP = sidx(sr, sc);
+  const unsigned char cl = S.cls[sP];
+  const bool wall = cl & C_WALL;
+  bool computed = false;
+  float o[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};  // of wall cells and outside: never written in the reference
+  if ((cl & C_INT) && !wall) {
+    const bool alldry = S.cls[sidx(sr - 1, sc)] & S.cls[sidx(sr + 1, sc)] & S.cls[sidx(sr, sc - 1)] &
+                        S.cls[sidx(sr, sc + 1)] & cl & C_DRY;
+    if (alldry) {
+      // all five cells dry: the reference returns before storing
+      // (solver_drydomain.cpp:60-76), so the fluxes of the last step that
+      // computed them stay in effect
+      const long long gi = fx_ix(d, irow, icol);
+      const float* rp = fx_rec(d, sprev + gi);
+      o[0] = rp[FX_R_FE1];
+      o[1] = d.fe2_f[gi];
+      o[2] = d.fe3_f[gi];
+      o[3] = rp[FX_R_FN1];
+      o[4] = d.fn2_f[gi];
+      o[5] = d.fn3_f[gi];
     } else {
-      solver_wet32(d, S, sr, scc, irow0 - 1 + fr, icol0 - 1 + fc, dtl, o);
-      for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
+      computed = true;
+      if (cl & C_DRY) solver_dry32(d, S, bed, sr, sc, irow, icol, dtl, o);
+      else solver_wet32(d, S, bed, sr, sc, irow, icol, dtl, o);
     }
   }
+  for (int j = 0; j < 3; ++j) S.f[j][tid] = o[3 + j];
+  float w[3];  // the west neighbour's east faces
+  for (int j = 0; j < 3; ++j) w[j] = __shfl_up_sync(0xffffffffu, o[j], 1);
   __syncthreads();
   bool wet = false;
   float c_eta = 0.f, c_lo = 0.f, c_qx = 0.f, c_qy = 0.f;  // this thread's cell after the update
   if (own) {
     const long long gi = fx_ix(d, irow, icol);
-    const int sP = sidx(lx + 2, ly + 2);
-    const int fP = (ly + 1) * FXN + (lx + 1), fW = (ly + 1) * FXN + lx, fS = ly * FXN + (lx + 1);
-    const unsigned char cl = S.cls[sP];
-    const bool wall = cl & C_WALL;
-    const int i4 = (ly + 2) * STG_W4 + lx + 2 + so.o4;
-    const uint8_t fl = stg ? stg[L::O_FL + (ly + 2) * STG_W1 + lx + 2 + so.o1] : d.flags[sprev + gi];
+    const int S0 = tid - BX;  // the south neighbour's north faces
+    const int i4 = sc * STG_W4 + sr + so.o4;
+    const uint8_t fl = STAGED ? stg[L::O_FL + sc * STG_W1 + sr + so.o1] : d.flags[sprev + gi];
     const float eta1 = S.eta[sP];
-    const float etapre = stg ? reinterpret_cast<const float*>(stg + L::O_Z)[i4] : d.eta[pprev + gi];
+    const float etapre = STAGED ? reinterpret_cast<const float*>(stg + L::O_Z)[i4] : d.eta[pprev + gi];
     float h0v = fmaxf(0.0f, etapre);
     double mi = 0.0;
     float hpv = 0.0f, miv = 0.0f;  // the record's pre-melt depth and melt depth
@@ -1309,7 +1334,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       bmelt = mi * d.arbase;
     }
     if (is_inflow(d, irow, icol)) {  // common.cpp:300-315 (h0 = the depth after the inflow)
-      float em = etapre, lm = stg ? reinterpret_cast<const float*>(stg + L::O_LO)[i4] : d.eta_lo[pprev + gi];
+      float em = etapre, lm = STAGED ? reinterpret_cast<const float*>(stg + L::O_LO)[i4] : d.eta_lo[pprev + gi];
       if (melt_on && !(fl & FX_F_NODATA)) fx_dd_add(em, lm, (float)mi);
       const double dm = fx_dd_val(em, lm);
       record_inflow_hm(d, c, fmax(dm, 0.0));
@@ -1319,18 +1344,16 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     if (!(cl & C_DRY)) d.twet_f[gi] += c.twet_f;
     float dh = 0.f, dqx = 0.f, dqy = 0.f, qxfP = 0.f, qyfP = 0.f;
     if (!wall) {
-      dh = (div_dxy_f(d, S.f[0][fW] - S.f[0][fP]) + div_dxy_f(d, S.f[3][fS] - S.f[3][fP])) * dtl;
-      dqx = (div_dxy_f(d, S.f[1][fW] - S.f[1][fP]) + div_dxy_f(d, S.f[4][fS] - S.f[4][fP])) * dtl;
-      dqy = (div_dxy_f(d, S.f[2][fW] - S.f[2][fP]) + div_dxy_f(d, S.f[5][fS] - S.f[5][fP])) * dtl;
-      qxfP = S.f[0][fP] * dtl;
-      qyfP = S.f[3][fP] * dtl;
-      const unsigned char clE = S.cls[sidx(lx + 3, ly + 2)], clN = S.cls[sidx(lx + 2, ly + 3)];
-      if (irow == d.nr || (clE & C_WALL)) bout += (double)S.f[0][fP] * d.dxy * c.dtfl;
-      if (icol == d.nc || (clN & C_WALL)) bout += (double)S.f[3][fP] * d.dxy * c.dtfl;
+      dh = (div_dxy_f(d, w[0] - o[0]) + div_dxy_f(d, S.f[0][S0] - o[3])) * dtl;
+      dqx = (div_dxy_f(d, w[1] - o[1]) + div_dxy_f(d, S.f[1][S0] - o[4])) * dtl;
+      dqy = (div_dxy_f(d, w[2] - o[2]) + div_dxy_f(d, S.f[2][S0] - o[5])) * dtl;
+      qxfP = o[0] * dtl;
+      qyfP = o[3] * dtl;
+      const unsigned char clE = S.cls[sidx(sr + 1, sc)], clN = S.cls[sidx(sr, sc + 1)];
+      if (irow == d.nr || (clE & C_WALL)) bout += (double)o[0] * d.dxy * c.dtfl;
+      if (icol == d.nc || (clN & C_WALL)) bout += (double)o[3] * d.dxy * c.dtfl;
     }
-    const unsigned char clW = S.cls[sidx(lx + 1, ly + 2)], clS = S.cls[sidx(lx + 2, ly + 1)];
-    const float qxfW = ((clW & (C_INT | C_WALL)) == C_INT) ? S.f[0][fW] * dtl : 0.0f;
-    const float qyfS = ((clS & (C_INT | C_WALL)) == C_INT) ? S.f[3][fS] * dtl : 0.0f;
+    const float qxfW = w[0] * dtl, qyfS = S.f[0][S0] * dtl;
     float eta = eta1, lo = S.eta_lo[sP];
     fx_dd_add(eta, lo, dh);
     const float h = fmaxf(0.0f, eta);
@@ -1362,21 +1385,14 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     d.qy_f[pcur + gi] = qy;
     const uint8_t fl1 = (fl & (FX_F_WALL | FX_F_NODATA)) | ((fl & FX_F_LDRY) ? FX_F_LDRY_PREV : 0) | ld;
     d.flags[scur + gi] = fl1;
-    float fe1v = 0.0f, fn1v = 0.0f;
-    if ((cl & C_INT) && !wall) {
-      const bool computed =
-          !(cl & C_DRY) || !(S.cls[sidx(lx + 1, ly + 2)] & S.cls[sidx(lx + 3, ly + 2)] &
-                              S.cls[sidx(lx + 2, ly + 1)] & S.cls[sidx(lx + 2, ly + 3)] & C_DRY);
-      fe1v = S.f[0][fP];
-      fn1v = S.f[3][fP];
-      if (computed && (d.store_all_fluxes || dd_le_hdry(d, eta, lo))) {
-        d.fe2_f[gi] = S.f[1][fP];
-        d.fe3_f[gi] = S.f[2][fP];
-        d.fn2_f[gi] = S.f[4][fP];
-        d.fn3_f[gi] = S.f[5][fP];
-      }
+    if (computed && (d.store_all_fluxes || dd_le_hdry(d, eta, lo))) {
+      d.fe2_f[gi] = o[1];
+      d.fe3_f[gi] = o[2];
+      d.fn2_f[gi] = o[4];
+      d.fn3_f[gi] = o[5];
     }
-    put_rec32(d, scur + gi, h0v, h, hpv, miv, fe1v, fn1v, fl1);
+    // fe_1 and fn_1 of every cell go to this step's slot, kept ones too
+    put_rec32(d, scur + gi, h0v, h, hpv, miv, o[0], o[3], fl1);
     wet = eta > 0.0f && !dd_le_hdry(d, eta, lo);
     c_eta = eta;
     c_lo = lo;
@@ -1389,11 +1405,57 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
   return true;
 }
 
-// The FP64 step of one tile (the reference's arithmetic, bit for bit).
+// A step without solver (no wet cell): the Courant scan and add_meteo only
+// (main.cpp:300-370, the solver block at :385 is skipped). The solute
+// dilution of add_meteo is applied by the ADE sweep (fx_ade.cu).
 template <int BY>
+__device__ __forceinline__ void idle_tile64(const fx_dev& d, const StepCtl& c, const fx_tile& tile, TilePart& acc) {
+  const int irow = 1 + tile.bx * TX + threadIdx.x, icol = 1 + tile.by * Tile<BY>::TY + threadIdx.y;
+  const bool own = threadIdx.x < TX && threadIdx.y < Tile<BY>::TY && irow <= d.nr && icol <= d.nc;
+  const bool melt_on = d.has_meteo != 0;
+  const long long sprev = c.sprev, scur = c.scur, pprev = c.pprev, pcur = c.pcur;
+  double dtc = __longlong_as_double(0x7ff0000000000000LL), hm = 0.0, bmelt = 0.0;
+  if (own) {
+    const long long gi = fx_ix(d, irow, icol);
+    const double zb = d.zb[gi], zpre = d.z[pprev + gi];
+    const uint8_t fl = d.flags[sprev + gi];
+    const double hpre = max0(zpre - zb);
+    uint8_t ld = hpre > d.hdry ? 0 : 1;  // Courant scan (:308-320)
+    double z1 = zpre, h1 = hpre, hpv = 0.0;
+    if (melt_on && zb != d.nodata) {
+      const double mi = melt_depth(d, c, gi);
+      bmelt = mi * d.arbase;
+      hpv = max0(zpre - zb);  // the dilution's hp (common.cpp:216)
+      z1 = zpre + mi;
+      h1 = max0(z1 - zb);
+      if (h1 <= d.hdry) ld = 0;  // common.cpp:219-222
+    }
+    if (is_inflow(d, irow, icol)) {  // common.cpp:300-315
+      const double zm = z1;
+      record_inflow_hm(d, c, max0(zm - zb));
+      z1 = inflow_z(z1, zb, c.inflowi);
+      h1 = max0(z1 - zb);
+      ld = h1 <= d.hdry ? 1 : 0;
+      bmelt += (z1 - zm) * d.arbase;
+    }
+    const double qx = d.qx[pprev + gi], qy = d.qy[pprev + gi];
+    d.z[pcur + gi] = z1;
+    d.qx[pcur + gi] = qx;
+    d.qy[pcur + gi] = qy;
+    const uint8_t fl1 = (fl & (FX_F_WALL | FX_F_NODATA)) | ((fl & FX_F_LDRY) ? FX_F_LDRY_PREV : 0) | ld;
+    d.flags[scur + gi] = fl1;
+    const double* rp = fx_rec64(d, sprev + gi);  // fluxes are unchanged by a step without solver
+    put_rec64(d, scur + gi, h1, h1, hpv, rp[FX_R64_FE1], rp[FX_R64_FN1], fl1);
+    courant_cell(d, h1, qx, qy, dtc, hm);
+  }
+  acc.add(dtc, hm, bmelt, 0.0);
+}
+
+// The FP64 step of one tile (the reference's arithmetic, bit for bit).
+template <int BY, bool STAGED>
 __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, const fx_tile& tile,
-                                             HydroSmem<BY>& S, TilePart& acc, const unsigned char* stg = nullptr,
-                                             int bad = 0) {
+                                             HydroSmem64<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad) {
+  using SM = HydroSmem64<BY, STAGED>;
   using L = StageLayout<false, BY>;
   const StageOff so = stage_off(tile.bx);
   constexpr int TY = Tile<BY>::TY, NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX;
@@ -1401,8 +1463,10 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   const int lx = threadIdx.x, ly = threadIdx.y;
   const int tid = ly * BX + lx;
   const int irow0 = 1 + tile.bx * TX, icol0 = 1 + tile.by * TY;
-  const int irow = irow0 + lx, icol = icol0 + ly;
-  const bool own = lx < TX && ly < TY && irow <= d.nr && icol <= d.nc;
+  // The thread's face-flux cell and, but for the west row and south column of
+  // the tile, the cell it owns.
+  const int irow = irow0 - 1 + lx, icol = icol0 - 1 + ly;
+  const bool own = lx > 0 && ly > 0 && irow <= d.nr && icol <= d.nc;
   const double dtl = c.dtfl;
   const bool melt_on = d.has_meteo != 0;
 
@@ -1412,50 +1476,13 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   // included, and writes the other.
   const long long sprev = c.sprev, scur = c.scur, pprev = c.pprev, pcur = c.pcur;
 
-  if (!c.active) {
-    // No wet cell: the step is the Courant scan plus add_meteo only
-    // (main.cpp:300-370, the solver block at :385 is skipped). The solute
-    // dilution of add_meteo is applied by the ADE sweep (fx_ade.cu).
-    double dtc = __longlong_as_double(0x7ff0000000000000LL), hm = 0.0, bmelt = 0.0;
-    if (own) {
-      const long long gi = fx_ix(d, irow, icol);
-      const double zb = d.zb[gi], zpre = d.z[pprev + gi];
-      const uint8_t fl = d.flags[sprev + gi];
-      const double hpre = max0(zpre - zb);
-      uint8_t ld = hpre > d.hdry ? 0 : 1;  // Courant scan (:308-320)
-      double z1 = zpre, h1 = hpre, hpv = 0.0;
-      if (melt_on && zb != d.nodata) {
-        const double mi = melt_depth(d, c, gi);
-        bmelt = mi * d.arbase;
-        hpv = max0(zpre - zb);  // the dilution's hp (common.cpp:216)
-        z1 = zpre + mi;
-        h1 = max0(z1 - zb);
-        if (h1 <= d.hdry) ld = 0;  // common.cpp:219-222
-      }
-      if (is_inflow(d, irow, icol)) {  // common.cpp:300-315
-        const double zm = z1;
-        record_inflow_hm(d, c, max0(zm - zb));
-        z1 = inflow_z(z1, zb, c.inflowi);
-        h1 = max0(z1 - zb);
-        ld = h1 <= d.hdry ? 1 : 0;
-        bmelt += (z1 - zm) * d.arbase;
-      }
-      const double qx = d.qx[pprev + gi], qy = d.qy[pprev + gi];
-      d.z[pcur + gi] = z1;
-      d.qx[pcur + gi] = qx;
-      d.qy[pcur + gi] = qy;
-      const uint8_t fl1 = (fl & (FX_F_WALL | FX_F_NODATA)) | ((fl & FX_F_LDRY) ? FX_F_LDRY_PREV : 0) | ld;
-      d.flags[scur + gi] = fl1;
-      const double* rp = fx_rec64(d, sprev + gi);  // fluxes are unchanged by a step without solver
-      put_rec64(d, scur + gi, h1, h1, hpv, rp[FX_R64_FE1], rp[FX_R64_FN1], fl1);
-      courant_cell(d, h1, qx, qy, dtc, hm);
-    }
-    acc.add(dtc, hm, bmelt, 0.0);
-    return true;
-  }
 
+  const auto bed = [&] {
+    if constexpr (STAGED) return Bed<STG_W8>{reinterpret_cast<const double*>(stg + L::O_ZB) + so.o8};
+    else return Bed<SX>{S.zb};
+  }();
   // ---- phase A: stencil load, melt, Loop 1 ---------------------------------
-  if (stg) {
+  if constexpr (STAGED) {
     // staged by TMA: the same values, read from shared memory
     const double* g_z = reinterpret_cast<const double*>(stg + L::O_Z);
     const double* g_zb = reinterpret_cast<const double*>(stg + L::O_ZB);
@@ -1476,8 +1503,11 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       if (r >= 1 && r <= d.nr && q >= 1 && q <= d.nc) {
         cl = C_INT;
         if (g_fl[sc * STG_W1 + sr + so.o1] & FX_F_WALL) cl |= C_WALL;
-        if (melt_on && zb != d.nodata)
-          z = z + (d.melt_mult ? over((double)c.meteo_rate * g_mm[i8], DAY_MM, 1.0 / DAY_MM) * c.dtfl : c.meteoi);
+        if (melt_on && zb != d.nodata) {
+          const double mi = d.melt_mult ? over((double)c.meteo_rate * g_mm[i8], DAY_MM, 1.0 / DAY_MM) * c.dtfl : c.meteoi;
+          S.mi[k] = mi;
+          z = z + mi;
+        }
         if (is_inflow(d, r, q)) z = inflow_z(z, zb, c.inflowi);
         const double h1 = max0(z - zb);
         if (h1 <= d.hdry) {
@@ -1487,53 +1517,53 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
         }
       }
       S.z[k] = z;
-      S.zb[k] = zb;
       S.qx[k] = qx;
       S.qy[k] = qy;
       S.cls[k] = cl;
-      if constexpr (HydroSmem<BY>::VEL) {
+      if constexpr (SM::VEL) {
         const Over den(at_least(at_least(max0(z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0));
         S.u[k] = den.of(qx);
         S.v[k] = den.of(qy);
       }
     }
-  } else
+  } else {
 #pragma unroll 1
-  for (int pass = 0; pass < 2; ++pass) {
-    int sr, sc;
-    if (!stencil_cell<BY>(pass, lx, ly, sr, sc)) break;
-    const int k = sidx(sr, sc);
-    const int r = irow0 - 2 + sr, q = icol0 - 2 + sc;
-    double z = 0.0, zb = 0.0, qx = 0.0, qy = 0.0;
-    unsigned char cl = 0;
-    if (r >= 0 && r <= d.nr + 1 && q >= 0 && q <= d.nc + 1) {
-      const long long gi = fx_ix(d, r, q);
-      z = d.z[pprev + gi];
-      zb = d.zb[gi];
-      qx = d.qx[pprev + gi];
-      qy = d.qy[pprev + gi];
-      if (r >= 1 && r <= d.nr && q >= 1 && q <= d.nc) {
-        cl = C_INT;
-        if (d.flags[sprev + gi] & FX_F_WALL) cl |= C_WALL;
-        if (melt_on && zb != d.nodata) z = z + melt_depth(d, c, gi);
-        if (is_inflow(d, r, q)) z = inflow_z(z, zb, c.inflowi);
-        const double h1 = max0(z - zb);
-        if (h1 <= d.hdry) {
-          qx = 0.0;
-          qy = 0.0;
-          cl |= C_DRY;
+    for (int pass = 0; pass < 2; ++pass) {
+      int sr, sc;
+      if (!stencil_cell<BY>(pass, lx, ly, sr, sc)) break;
+      const int k = sidx(sr, sc);
+      const int r = irow0 - 2 + sr, q = icol0 - 2 + sc;
+      double z = 0.0, zb = 0.0, qx = 0.0, qy = 0.0;
+      unsigned char cl = 0;
+      if (r >= 0 && r <= d.nr + 1 && q >= 0 && q <= d.nc + 1) {
+        const long long gi = fx_ix(d, r, q);
+        z = d.z[pprev + gi];
+        zb = d.zb[gi];
+        qx = d.qx[pprev + gi];
+        qy = d.qy[pprev + gi];
+        if (r >= 1 && r <= d.nr && q >= 1 && q <= d.nc) {
+          cl = C_INT;
+          if (d.flags[sprev + gi] & FX_F_WALL) cl |= C_WALL;
+          if (melt_on && zb != d.nodata) z = z + melt_depth(d, c, gi);
+          if (is_inflow(d, r, q)) z = inflow_z(z, zb, c.inflowi);
+          const double h1 = max0(z - zb);
+          if (h1 <= d.hdry) {
+            qx = 0.0;
+            qy = 0.0;
+            cl |= C_DRY;
+          }
         }
       }
-    }
-    S.z[k] = z;
-    S.zb[k] = zb;
-    S.qx[k] = qx;
-    S.qy[k] = qy;
-    S.cls[k] = cl;
-    if constexpr (HydroSmem<BY>::VEL) {
-      const Over den(at_least(at_least(max0(z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0));
-      S.u[k] = den.of(qx);
-      S.v[k] = den.of(qy);
+      S.z[k] = z;
+      S.zb[k] = zb;
+      S.qx[k] = qx;
+      S.qy[k] = qy;
+      S.cls[k] = cl;
+      if constexpr (SM::VEL) {
+        const Over den(at_least(at_least(max0(z - zb), d.hdry), (cl & C_INT) ? d.ks : 0.0));
+        S.u[k] = den.of(qx);
+        S.v[k] = den.of(qy);
+      }
     }
   }
   // the stencil is complete; a thread whose stage wait gave up (bad) stops
@@ -1545,37 +1575,38 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   // wet, dry and kept cells, which would fill the warps with one kind each,
   // cost a pass and a barrier more than the divergence they avoid: 2048 x 2048
   // cells and a 384 x 384 basin take the same time without, 1000 x 700 cells 1 % less.
-  {
-    const int k = tid, fr = lx, fc = ly;
-    const int sr = fr + 1, sc = fc + 1;
-    const unsigned char cl = S.cls[sidx(sr, sc)];
-    double o[6];
-    if (!(cl & C_INT) || (cl & C_WALL)) {
-      for (int j = 0; j < 6; ++j) S.f[j][k] = 0.0;  // never written in the reference
-    } else if (cl & C_DRY) {
+  // Its six fluxes stay in registers for the update of the cell itself; the
+  // east faces' go to the neighbour's lane by shuffle, the north faces' to the
+  // next column's warp through shared memory.
+  const int sr = lx + 1, sc = ly + 1, sP = sidx(sr, sc);
+  const unsigned char cl = S.cls[sP];
+  const bool wall = cl & C_WALL;
+  bool computed = false;
+  double o[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // of wall cells and outside: never written in the reference
+  if ((cl & C_INT) && !wall) {
+    const bool alldry = S.cls[sidx(sr - 1, sc)] & S.cls[sidx(sr + 1, sc)] & S.cls[sidx(sr, sc - 1)] &
+                        S.cls[sidx(sr, sc + 1)] & cl & C_DRY;
+    if (alldry) {
       // all five cells dry: the reference returns before storing
       // (solver_drydomain.cpp:60-76), so the fluxes of the last step that
       // computed them stay in effect
-      const bool alldry = S.cls[sidx(sr - 1, sc)] & S.cls[sidx(sr + 1, sc)] & S.cls[sidx(sr, sc - 1)] &
-                          S.cls[sidx(sr, sc + 1)] & C_DRY;
-      if (alldry) {
-        const long long gi = fx_ix(d, irow0 - 1 + fr, icol0 - 1 + fc);
-        const double* rp = fx_rec64(d, sprev + gi);
-        S.f[0][k] = rp[FX_R64_FE1];
-        S.f[1][k] = d.fe2[gi];
-        S.f[2][k] = d.fe3[gi];
-        S.f[3][k] = rp[FX_R64_FN1];
-        S.f[4][k] = d.fn2[gi];
-        S.f[5][k] = d.fn3[gi];
-      } else {
-        solver_dry(d, S, sr, sc, irow0 - 1 + fr, icol0 - 1 + fc, dtl, o);
-        for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
-      }
+      const long long gi = fx_ix(d, irow, icol);
+      const double* rp = fx_rec64(d, sprev + gi);
+      o[0] = rp[FX_R64_FE1];
+      o[1] = d.fe2[gi];
+      o[2] = d.fe3[gi];
+      o[3] = rp[FX_R64_FN1];
+      o[4] = d.fn2[gi];
+      o[5] = d.fn3[gi];
     } else {
-      solver_wet(d, S, sr, sc, irow0 - 1 + fr, icol0 - 1 + fc, c.dt, o);
-      for (int j = 0; j < 6; ++j) S.f[j][k] = o[j];
+      computed = true;
+      if (cl & C_DRY) solver_dry(d, S, bed, sr, sc, irow, icol, dtl, o);
+      else solver_wet(d, S, bed, sr, sc, irow, icol, c.dt, o);
     }
   }
+  for (int j = 0; j < 3; ++j) S.f[j][tid] = o[3 + j];
+  double w[3];  // the west neighbour's east faces
+  for (int j = 0; j < 3; ++j) w[j] = __shfl_up_sync(0xffffffffu, o[j], 1);
   __syncthreads();
 
   // ---- phase D: Loop 3, Loop 4, friction, store, next Courant --------------
@@ -1583,15 +1614,12 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   double c_h = 0.0, c_qx = 0.0, c_qy = 0.0;  // this thread's cell after the update
   if (own) {
     const long long gi = fx_ix(d, irow, icol);
-    const int sP = sidx(lx + 2, ly + 2);
-    const int fP = (ly + 1) * FXN + (lx + 1), fW = (ly + 1) * FXN + lx, fS = ly * FXN + (lx + 1);
-    const unsigned char cl = S.cls[sP];
-    const bool wall = cl & C_WALL;
-    const int i8 = (ly + 2) * STG_W8 + lx + 2 + so.o8;
-    const uint8_t fl = stg ? stg[L::O_FL + (ly + 2) * STG_W1 + lx + 2 + so.o1] : d.flags[sprev + gi];
-    const double zb = S.zb[sP];
+    const int S0 = tid - BX;  // the south neighbour's north faces
+    const int i8 = sc * STG_W8 + sr + so.o8;
+    const uint8_t fl = STAGED ? stg[L::O_FL + sc * STG_W1 + sr + so.o1] : d.flags[sprev + gi];
+    const double zb = bed(sr, sc);
     const double z1 = S.z[sP];
-    const double zpre = stg ? reinterpret_cast<const double*>(stg + L::O_Z)[i8] : d.z[pprev + gi];
+    const double zpre = STAGED ? reinterpret_cast<const double*>(stg + L::O_Z)[i8] : d.z[pprev + gi];
 
     // add_meteo's h0 (common.cpp:223): the depth after the melt, or the
     // Courant scan's copy of h (main.cpp:305) for cells it skips. Its solute
@@ -1601,9 +1629,7 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     if (melt_on && zb != d.nodata) {
       h0v = max0(z1 - zb);
       hpv = max0(zpre - zb);  // the dilution's hp (common.cpp:216)
-      mi = (stg && d.melt_mult)
-               ? over((double)c.meteo_rate * reinterpret_cast<const double*>(stg + L::O_MM)[i8], DAY_MM, 1.0 / DAY_MM) * c.dtfl
-               : melt_depth(d, c, gi);
+      mi = STAGED ? S.mi[sP] : melt_depth(d, c, gi);
       bmelt = mi * d.arbase;
     }
     if (is_inflow(d, irow, icol)) {  // common.cpp:300-315 (h0 = the depth after the inflow)
@@ -1618,22 +1644,20 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     // Loop 3 (:93-120)
     double dh = 0.0, dqx = 0.0, dqy = 0.0, qxfP = 0.0, qyfP = 0.0;
     if (!wall) {
-      dh = (div_dxy(d, S.f[0][fW] - S.f[0][fP]) + div_dxy(d, S.f[3][fS] - S.f[3][fP])) * dtl;
-      dqx = (div_dxy(d, S.f[1][fW] - S.f[1][fP]) + div_dxy(d, S.f[4][fS] - S.f[4][fP])) * dtl;
-      dqy = (div_dxy(d, S.f[2][fW] - S.f[2][fP]) + div_dxy(d, S.f[5][fS] - S.f[5][fP])) * dtl;
-      qxfP = S.f[0][fP] * dtl;
-      qyfP = S.f[3][fP] * dtl;
+      dh = (div_dxy(d, w[0] - o[0]) + div_dxy(d, S.f[0][S0] - o[3])) * dtl;
+      dqx = (div_dxy(d, w[1] - o[1]) + div_dxy(d, S.f[1][S0] - o[4])) * dtl;
+      dqy = (div_dxy(d, w[2] - o[2]) + div_dxy(d, S.f[2][S0] - o[5])) * dtl;
+      qxfP = o[0] * dtl;
+      qyfP = o[3] * dtl;
     }
-    const unsigned char clW = S.cls[sidx(lx + 1, ly + 2)], clS = S.cls[sidx(lx + 2, ly + 1)];
     if (!wall) {
       // water leaving the domain this step: through the outflow faces, and
       // into wall cells (which never take it up, hydrodynamics_calc.cpp:111-117)
-      const unsigned char clE = S.cls[sidx(lx + 3, ly + 2)], clN = S.cls[sidx(lx + 2, ly + 3)];
-      if (irow == d.nr || (clE & C_WALL)) bout += S.f[0][fP] * d.dxy * dtl;
-      if (icol == d.nc || (clN & C_WALL)) bout += S.f[3][fP] * d.dxy * dtl;
+      const unsigned char clE = S.cls[sidx(sr + 1, sc)], clN = S.cls[sidx(sr, sc + 1)];
+      if (irow == d.nr || (clE & C_WALL)) bout += o[0] * d.dxy * dtl;
+      if (icol == d.nc || (clN & C_WALL)) bout += o[3] * d.dxy * dtl;
     }
-    const double qxfW = ((clW & (C_INT | C_WALL)) == C_INT) ? S.f[0][fW] * dtl : 0.0;
-    const double qyfS = ((clS & (C_INT | C_WALL)) == C_INT) ? S.f[3][fS] * dtl : 0.0;
+    const double qxfW = w[0] * dtl, qyfS = S.f[0][S0] * dtl;
 
     // Loop 4 (:123-154)
     const double z = z1 + dh;
@@ -1673,24 +1697,14 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     // ends the step wet (h > hdry) is wet again at the next solver step as
     // long as forcing adds water, so those three-quarters of the flux
     // traffic are skipped for it.
-    const unsigned char clP = cl;
-    double fe1v = 0.0, fn1v = 0.0;
-    if ((clP & C_INT) && !(clP & C_WALL)) {
-      const bool computed =
-          !(clP & C_DRY) || !(S.cls[sidx(lx + 1, ly + 2)] & S.cls[sidx(lx + 3, ly + 2)] &
-                              S.cls[sidx(lx + 2, ly + 1)] & S.cls[sidx(lx + 2, ly + 3)] & C_DRY);
-      // fe_1/fn_1 of every cell go to this step's slot: computed ones, or the
-      // stale ones carried over (already in S.f for stale cells).
-      fe1v = S.f[0][fP];
-      fn1v = S.f[3][fP];
-      if (computed && (d.store_all_fluxes || !(h > d.hdry))) {
-        d.fe2[gi] = S.f[1][fP];
-        d.fe3[gi] = S.f[2][fP];
-        d.fn2[gi] = S.f[4][fP];
-        d.fn3[gi] = S.f[5][fP];
-      }
-    }  // walls: fe_1 = fn_1 = 0, never written in the reference
-    put_rec64(d, scur + gi, h0v, h, hpv, fe1v, fn1v, fl1);
+    if (computed && (d.store_all_fluxes || !(h > d.hdry))) {
+      d.fe2[gi] = o[1];
+      d.fe3[gi] = o[2];
+      d.fn2[gi] = o[4];
+      d.fn3[gi] = o[5];
+    }
+    // fe_1 and fn_1 of every cell go to this step's slot, kept ones too
+    put_rec64(d, scur + gi, h0v, h, hpv, o[0], o[3], fl1);
     c_h = h;
     c_qx = qx;
     c_qy = qy;
@@ -1704,9 +1718,23 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
 // Reads the step's fields of the control block (written by k_finalize) into
 // shared memory, then runs the tile in the domain's precision.
 template <bool P32, int BY>
-__device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile, HydroSmem<BY>& S,
+__device__ __forceinline__ void idle_tile(const fx_dev& d, const StepCtl& c, const fx_tile& tile, TilePart& acc) {
+  if constexpr (P32) idle_tile32<BY>(d, c, tile, acc);
+  else idle_tile64<BY>(d, c, tile, acc);
+}
+// One tile's step. STAGED: its stencil is in the stage at `stg`, else it is
+// read from global memory. `bad`: this thread's wait for the stage gave up.
+template <bool P32, int BY, bool STAGED>
+__device__ __forceinline__ bool hydro_tile(const fx_dev& d, const StepCtl& c, const fx_tile& tile,
+                                           HydroSmem<P32, BY, STAGED>& S, TilePart& acc, const unsigned char* stg,
+                                           int bad) {
+  if constexpr (P32) return hydro_tile32<BY, STAGED>(d, c, tile, S, acc, stg, bad);
+  else return hydro_tile64<BY, STAGED>(d, c, tile, S, acc, stg, bad);
+}
+
+template <bool P32, int BY>
+__device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile, HydroSmem<P32, BY, false>& S,
                                             StepCtl& sc) {
-  static_assert(sizeof(HydroSmem32<BY>) <= sizeof(HydroSmem<BY>), "FP32 tile state reuses the FP64 one");
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     read_ctl(d, sc);
   }
@@ -1714,8 +1742,8 @@ __device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile
   const StepCtl c = sc;
   if (!c.live) return;
   TilePart acc = tile_part();
-  if constexpr (P32) hydro_tile32<BY>(d, c, tile, *reinterpret_cast<HydroSmem32<BY>*>(&S), acc);
-  else hydro_tile64<BY>(d, c, tile, S, acc);
+  if (!c.active) idle_tile<P32, BY>(d, c, tile, acc);
+  else hydro_tile<P32, BY, false>(d, c, tile, S, acc, nullptr, 0);
   reduce_part(d, S, acc);
 }
 
@@ -1736,7 +1764,7 @@ constexpr int min_blocks() { return (P32 ? 32 : BY == 4 ? 20 : 24) / BY; }
 // fields are instruction operands. Block (x, y) is tile (x, y).
 template <bool P32, int BY>
 __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>()) k_hydro_one(const __grid_constant__ fx_dev d) {
-  __shared__ HydroSmem<BY> S;
+  __shared__ HydroSmem<P32, BY, false> S;
   __shared__ StepCtl sc;
   const fx_tile tile{0, (int)blockIdx.x, (int)blockIdx.y, 0};
   hydro_block<P32, BY>(d, tile, S, sc);
@@ -1747,7 +1775,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>()) k_hydro_one(co
 template <bool P32, int BY>
 __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>()) k_hydro_batch(const fx_dev* __restrict__ devs,
                                                                         const fx_tile* __restrict__ tiles) {
-  __shared__ HydroSmem<BY> S;
+  __shared__ HydroSmem<P32, BY, false> S;
   __shared__ fx_dev sd;
   __shared__ StepCtl sc;
   const fx_tile tile = tiles[blockIdx.x];
@@ -1832,16 +1860,14 @@ template <bool P32, int BY>
 __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
     k_hydro_tma(const __grid_constant__ fx_dev d, const __grid_constant__ fx_tmaps tm, int ntx, int nty) {
   using L = StageLayout<P32, BY>;
-  __shared__ HydroSmem<BY> S;
+  __shared__ HydroSmem<P32, BY, true> S;
   __shared__ StepCtl sc;
   __shared__ __align__(8) unsigned long long bar[2];
   extern __shared__ __align__(128) unsigned char dyn[];
   unsigned char* stage0 = dyn + ((128 - (smem_u32(dyn) & 127)) & 127);
   const int tid = threadIdx.y * BX + threadIdx.x;
   const int ntiles = ntx * nty;
-  if (tid == 0) {
-    read_ctl(d, sc);
-  }
+  if (tid == 0) read_ctl(d, sc);
   __syncthreads();
   const StepCtl c = sc;
   if (!c.live) return;
@@ -1849,9 +1875,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
   if (!c.active) {  // no solver this step: cell-local work only, nothing to stage
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
       const fx_tile tile{0, t % ntx, t / ntx, 0};
-      if constexpr (P32) hydro_tile32<BY>(d, c, tile, *reinterpret_cast<HydroSmem32<BY>*>(&S), acc);
-      else hydro_tile64<BY>(d, c, tile, S, acc);
-      __syncthreads();
+      idle_tile<P32, BY>(d, c, tile, acc);
     }
     reduce_part(d, S, acc);
     return;
@@ -1865,6 +1889,11 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
   __syncthreads();
   unsigned parity = 0u;  // bit q: phase of stage q's barrier
   int st = 0;
+  // the block's tiles are gridDim.x apart in the row-major order: in FP32 bx,
+  // by step along without a division (1 % of the kernel); in FP64 the
+  // registers this takes cost as much
+  int bx = blockIdx.x % ntx, by = blockIdx.x / ntx;
+  const int dbx = gridDim.x % ntx, dby = gridDim.x / ntx;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int tn = t + gridDim.x;
     if (tid == 0 && tn < ntiles)
@@ -1881,12 +1910,15 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
       }
     }
     parity ^= 1u << st;
-    const fx_tile tile{0, t % ntx, t / ntx, 0};
-    bool done;
-    if constexpr (P32)
-      done = hydro_tile32<BY>(d, c, tile, *reinterpret_cast<HydroSmem32<BY>*>(&S), acc, stage0 + st * L::BYTES, bad);
-    else done = hydro_tile64<BY>(d, c, tile, S, acc, stage0 + st * L::BYTES, bad);
-    if (!done) {  // every thread of the block takes this branch
+    const fx_tile tile = P32 ? fx_tile{0, bx, by, 0} : fx_tile{0, t % ntx, t / ntx, 0};
+    bx += dbx;
+    by += dby;
+    if (bx >= ntx) {
+      bx -= ntx;
+      ++by;
+    }
+    if (!hydro_tile<P32, BY, true>(d, c, tile, S, acc, stage0 + st * L::BYTES, bad)) {
+      // every thread of the block takes this branch
       if (tid == 0) {
         atomicCAS(&d.ctl->error, 0, FX_DEVERR_WAIT_TIMEOUT);
         // let the copy of the next tile, if one was issued, land before the block exits
@@ -1941,7 +1973,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
     k_hydro_batch_tma(const fx_dev* __restrict__ devs, const fx_tmaps* __restrict__ tms,
                       const fx_tile* __restrict__ tiles, int ntiles) {
   using L = StageLayout<P32, BY>;
-  __shared__ HydroSmem<BY> S;
+  __shared__ HydroSmem<P32, BY, true> S;
   __shared__ fx_dev sd;
   __shared__ StepCtl sc;
   __shared__ __align__(8) unsigned long long bar[2];
@@ -2011,9 +2043,9 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
     const StepCtl c = sc;
     if (c.live) {
       const fx_tile tile{0, tl.bx, tl.by, 0};
-      const unsigned char* stg = mine ? stage0 + st * L::BYTES : nullptr;
-      if constexpr (P32) hydro_tile32<BY>(sd, c, tile, *reinterpret_cast<HydroSmem32<BY>*>(&S), acc, stg);
-      else hydro_tile64<BY>(sd, c, tile, S, acc, stg);
+      // a domain that runs the solver this step was staged (batch_stage)
+      if (!c.active) idle_tile<P32, BY>(sd, c, tile, acc);
+      else hydro_tile<P32, BY, true>(sd, c, tile, S, acc, stage0 + st * L::BYTES, 0);
     }
     __syncthreads();  // the stage is free for the copy issued next iteration
     st ^= 1;
@@ -2027,7 +2059,7 @@ template <int BY>
 __global__ void __launch_bounds__(BX * BY) k_courant_scan(const fx_dev* __restrict__ devs,
                                                          const fx_tile* __restrict__ tiles) {
   constexpr int TY = Tile<BY>::TY;
-  __shared__ HydroSmem<BY> S;
+  __shared__ HydroSmem64<BY, true> S;
   __shared__ fx_dev sd;
   const fx_tile tile = tiles[blockIdx.x];
   if (threadIdx.x == 0 && threadIdx.y == 0) sd = devs[tile.dom];
