@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "fx_common.cuh"
+#include "fx_div.cuh"
 
 namespace fx {
 
@@ -86,47 +87,6 @@ __device__ __forceinline__ double fx_pow15(double h) {
   return p + (pe + h * slo);
 }
 
-// Quotients over a shared denominator, the bits of a / b: y = 1 / b, correctly
-// rounded, then two Newton corrections of a * y. The first leaves a faithful
-// quotient, so by Markstein's theorem (IBM J. Res. Dev. 34, 1990; Muller et al.,
-// Handbook of Floating-Point Arithmetic, ch. 4) the second rounds correctly; its
-// residual is exact for |a| >= 2^-700 and b, a below 2^200, 2^700. Anything else
-// divides, except 0, whose quotient is a * y (an FP64 division of 0 takes 436
-// cycles against 146 of an ordinary one, measured, and dry and resting cells
-// divide 0 all the time). The division stays out of line: a dozen copies of it
-// in the kernel cost more in instruction fetches than the quotients save
-// (2048 x 2048 cells 0.82 ms a step with them inline, 0.70 ms without, 0.80 ms
-// with plain divisions).
-__device__ __noinline__ double plain_div(double a, double b) { return a / b; }
-struct Over {
-  double b, y;
-  bool ok;
-  Over() = default;
-  __device__ __forceinline__ explicit Over(double b_) : b(b_), y(1.0 / b_) {
-    ok = (b > 6.223015277861142e-61) & (b < 1.6069380442589903e60);  // 2^-200, 2^200
-  }
-  __device__ __forceinline__ double of(double a) const {
-    const double q0 = a * y;
-    const double q1 = fma(fma(-b, q0, a), y, q0);
-    double q = fma(fma(-b, q1, a), y, q1);
-    const unsigned e = (unsigned)(__double2hiint(a) & 0x7ff00000) - ((1023u - 700u) << 20);
-    const bool zero = a == 0.0;
-    q = zero ? q0 : q;
-    if (!ok | ((e >= (1400u << 20)) & !zero)) q = plain_div(a, b);
-    return q;
-  }
-};
-// The same over a constant between 2^-200 and 2^200.
-__device__ __forceinline__ double over(double a, double b, double y) {
-  const double q0 = a * y;
-  const double q1 = fma(fma(-b, q0, a), y, q0);
-  double q = fma(fma(-b, q1, a), y, q1);
-  const unsigned e = (unsigned)(__double2hiint(a) & 0x7ff00000) - ((1023u - 700u) << 20);
-  const bool zero = a == 0.0;
-  q = zero ? q0 : q;
-  if ((e >= (1400u << 20)) & !zero) q = plain_div(a, b);
-  return q;
-}
 // x / dxy of the FP64 state. Out of line for the same reason; at a spacing of
 // 3, 1000 x 700 cells took 131 us a step with plain divisions, 112 us so.
 __device__ __noinline__ double over_dxy(double x, double dxy, double inv) { return over(x, dxy, inv); }
@@ -1159,9 +1119,9 @@ __device__ __forceinline__ void idle_tile32(const fx_dev& d, const StepCtl& c, c
   acc.add(dtc, hm, bmelt, 0.0);
 }
 
-template <int BY, bool STAGED>
+template <int BY, bool STAGED, class F>
 __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, const fx_tile& tile,
-                                             HydroSmem32<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad) {
+                                             HydroSmem32<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad, F stage_free) {
   using L = StageLayout<true, BY>;
   const StageOff so = stage_off(tile.bx);
   constexpr int TY = Tile<BY>::TY, NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX;
@@ -1313,35 +1273,52 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
   for (int j = 0; j < 3; ++j) S.f[j][tid] = o[3 + j];
   float w[3];  // the west neighbour's east faces
   for (int j = 0; j < 3; ++j) w[j] = __shfl_up_sync(0xffffffffu, o[j], 1);
-  __syncthreads();
-  bool wet = false;
-  float c_eta = 0.f, c_lo = 0.f, c_qx = 0.f, c_qy = 0.f;  // this thread's cell after the update
+  // What the update takes from the stage and the stencil is read here, before
+  // the barrier: after it the stage is free for the tile after next, and a
+  // warp that is done with its update may read the next tile's stencil while
+  // others are still at it, so a tile has two barriers. The wet time and the
+  // roughness are loaded here for the update behind the barrier: 4096 x 4096
+  // cells 0.92 ms a step before, 0.91 with two barriers, 0.86 with the loads.
+  bool wet = false, outE = false, outN = false;
+  uint8_t fl = 0;
+  float eta = 0.f, lo = 0.f, qx = 0.f, qy = 0.f;  // this thread's cell, before and after the update
+  float tw = 0.f, n = 0.f;
+  float h0v = 0.f, hpv = 0.f, miv = 0.f;          // the record's depths: at the start of the step, pre-melt, of the melt
   if (own) {
-    const long long gi = fx_ix(d, irow, icol);
-    const int S0 = tid - BX;  // the south neighbour's north faces
     const int i4 = sc * STG_W4 + sr + so.o4;
-    const uint8_t fl = STAGED ? stg[L::O_FL + sc * STG_W1 + sr + so.o1] : d.flags[sprev + gi];
-    const float eta1 = S.eta[sP];
+    const long long gi = fx_ix(d, irow, icol);
+    fl = STAGED ? stg[L::O_FL + sc * STG_W1 + sr + so.o1] : d.flags[sprev + gi];
+    if (!(cl & C_DRY)) tw = d.twet_f[gi];
+    if (d.manning_f) n = d.manning_f[gi];
+    eta = S.eta[sP];
+    lo = S.eta_lo[sP];
+    qx = S.qx[sP];
+    qy = S.qy[sP];
+    outE = irow == d.nr || (S.cls[sidx(sr + 1, sc)] & C_WALL);
+    outN = icol == d.nc || (S.cls[sidx(sr, sc + 1)] & C_WALL);
     const float etapre = STAGED ? reinterpret_cast<const float*>(stg + L::O_Z)[i4] : d.eta[pprev + gi];
-    float h0v = fmaxf(0.0f, etapre);
-    double mi = 0.0;
-    float hpv = 0.0f, miv = 0.0f;  // the record's pre-melt depth and melt depth
+    h0v = fmaxf(0.0f, etapre);
     if (melt_on && !(fl & FX_F_NODATA)) {
-      h0v = fmaxf(eta1, 0.0f);
+      h0v = fmaxf(eta, 0.0f);
       hpv = fmaxf(etapre, 0.0f);
       miv = S.mi[sP];
-      mi = (double)miv;
-      bmelt = mi * d.arbase;
+      bmelt = (double)miv * d.arbase;
     }
     if (is_inflow(d, irow, icol)) {  // common.cpp:300-315 (h0 = the depth after the inflow)
       float em = etapre, lm = STAGED ? reinterpret_cast<const float*>(stg + L::O_LO)[i4] : d.eta_lo[pprev + gi];
-      if (melt_on && !(fl & FX_F_NODATA)) fx_dd_add(em, lm, (float)mi);
+      if (melt_on && !(fl & FX_F_NODATA)) fx_dd_add(em, lm, miv);
       const double dm = fx_dd_val(em, lm);
       record_inflow_hm(d, c, fmax(dm, 0.0));
-      bmelt += (fx_dd_val(eta1, S.eta_lo[sP]) - dm) * d.arbase;
-      h0v = fmaxf(eta1, 0.0f);
+      bmelt += (fx_dd_val(eta, lo) - dm) * d.arbase;
+      h0v = fmaxf(eta, 0.0f);
     }
-    if (!(cl & C_DRY)) d.twet_f[gi] += c.twet_f;
+  }
+  __syncthreads();
+  stage_free();
+  if (own) {
+    const long long gi = fx_ix(d, irow, icol);
+    const int S0 = tid - BX;  // the south neighbour's north faces
+    if (!(cl & C_DRY)) d.twet_f[gi] = tw + c.twet_f;
     float dh = 0.f, dqx = 0.f, dqy = 0.f, qxfP = 0.f, qyfP = 0.f;
     if (!wall) {
       dh = (div_dxy_f(d, w[0] - o[0]) + div_dxy_f(d, S.f[0][S0] - o[3])) * dtl;
@@ -1349,28 +1326,24 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
       dqy = (div_dxy_f(d, w[2] - o[2]) + div_dxy_f(d, S.f[2][S0] - o[5])) * dtl;
       qxfP = o[0] * dtl;
       qyfP = o[3] * dtl;
-      const unsigned char clE = S.cls[sidx(sr + 1, sc)], clN = S.cls[sidx(sr, sc + 1)];
-      if (irow == d.nr || (clE & C_WALL)) bout += (double)o[0] * d.dxy * c.dtfl;
-      if (icol == d.nc || (clN & C_WALL)) bout += (double)o[3] * d.dxy * c.dtfl;
+      if (outE) bout += (double)o[0] * d.dxy * c.dtfl;
+      if (outN) bout += (double)o[3] * d.dxy * c.dtfl;
     }
     const float qxfW = w[0] * dtl, qyfS = S.f[0][S0] * dtl;
-    float eta = eta1, lo = S.eta_lo[sP];
     fx_dd_add(eta, lo, dh);
     const float h = fmaxf(0.0f, eta);
-    float qx, qy;
     uint8_t ld;
     if (dd_lt_hdry(d, eta, lo) || wall) {
       qx = qy = 0.0f;
       ld = 1;
     } else {
-      qx = S.qx[sP] + dqx;
-      qy = S.qy[sP] + dqy;
+      qx += dqx;
+      qy += dqy;
       qx = .1f * qxfW + .8f * qx + .1f * qxfP;
       qy = .1f * qyfS + .8f * qy + .1f * qyfP;
       ld = 0;
     }
     if (d.manning_f && ld == 0 && !wall) {
-      const float n = d.manning_f[gi];
       if (n != 0.0f) {
         const float qm = fsqrt(qx * qx + qy * qy);
         const float den = 1.0f + fdiv(dtl * d.f.gaccl * n * n * qm, h * h * fcbrt(h));
@@ -1394,12 +1367,8 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     // fe_1 and fn_1 of every cell go to this step's slot, kept ones too
     put_rec32(d, scur + gi, h0v, h, hpv, miv, o[0], o[3], fl1);
     wet = eta > 0.0f && !dd_le_hdry(d, eta, lo);
-    c_eta = eta;
-    c_lo = lo;
-    c_qx = qx;
-    c_qy = qy;
   }
-  courant_tile32(d, wet, c_eta, c_lo, c_qx, c_qy, acc);
+  courant_tile32(d, wet, eta, lo, qx, qy, acc);
   acc.melt += bmelt;
   acc.out += bout;
   return true;
@@ -1452,9 +1421,9 @@ __device__ __forceinline__ void idle_tile64(const fx_dev& d, const StepCtl& c, c
 }
 
 // The FP64 step of one tile (the reference's arithmetic, bit for bit).
-template <int BY, bool STAGED>
+template <int BY, bool STAGED, class F>
 __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, const fx_tile& tile,
-                                             HydroSmem64<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad) {
+                                             HydroSmem64<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad, F stage_free) {
   using SM = HydroSmem64<BY, STAGED>;
   using L = StageLayout<false, BY>;
   const StageOff so = stage_off(tile.bx);
@@ -1607,25 +1576,40 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   for (int j = 0; j < 3; ++j) S.f[j][tid] = o[3 + j];
   double w[3];  // the west neighbour's east faces
   for (int j = 0; j < 3; ++j) w[j] = __shfl_up_sync(0xffffffffu, o[j], 1);
-  __syncthreads();
-
-  // ---- phase D: Loop 3, Loop 4, friction, store, next Courant --------------
+  // ---- what the update takes from the stage and the stencil, read before the
+  // barrier: after it the stage is free for the tile after next, and a warp
+  // that is done with its update may read the next tile's stencil while others
+  // are still at it, so a tile has two barriers. The wet time and the roughness
+  // are loaded here for the update behind it: 2048 x 2048 cells 0.607 ms a step
+  // with three barriers and without the early loads, 0.584 so.
   double bmelt = 0.0, bout = 0.0;
-  double c_h = 0.0, c_qx = 0.0, c_qy = 0.0;  // this thread's cell after the update
+  double c_h = 0.0;  // this thread's depth after the update
+  bool outE = false, outN = false;
+  uint8_t fl = 0;
+  double zb = 0.0, z1 = 0.0, qx = 0.0, qy = 0.0;  // this thread's cell
+  double tw = 0.0, n = 0.0;
+  double h0v = 0.0, hpv = 0.0;                    // the record's depths
   if (own) {
     const long long gi = fx_ix(d, irow, icol);
-    const int S0 = tid - BX;  // the south neighbour's north faces
     const int i8 = sc * STG_W8 + sr + so.o8;
-    const uint8_t fl = STAGED ? stg[L::O_FL + sc * STG_W1 + sr + so.o1] : d.flags[sprev + gi];
-    const double zb = bed(sr, sc);
-    const double z1 = S.z[sP];
+    fl = STAGED ? stg[L::O_FL + sc * STG_W1 + sr + so.o1] : d.flags[sprev + gi];
+    if (!(cl & C_DRY)) tw = d.twet[gi];
+    if (d.manning) n = d.manning[gi];
+    zb = bed(sr, sc);
+    z1 = S.z[sP];
+    qx = S.qx[sP];
+    qy = S.qy[sP];
+    // water leaves the domain through the outflow faces, and into wall cells
+    // (which never take it up, hydrodynamics_calc.cpp:111-117)
+    outE = irow == d.nr || (S.cls[sidx(sr + 1, sc)] & C_WALL);
+    outN = icol == d.nc || (S.cls[sidx(sr, sc + 1)] & C_WALL);
     const double zpre = STAGED ? reinterpret_cast<const double*>(stg + L::O_Z)[i8] : d.z[pprev + gi];
 
     // add_meteo's h0 (common.cpp:223): the depth after the melt, or the
     // Courant scan's copy of h (main.cpp:305) for cells it skips. Its solute
     // dilution (:226-234) is applied by the ADE sweep (fx_ade.cu).
-    double h0v = max0(zpre - zb);
-    double mi = 0.0, hpv = 0.0;
+    h0v = max0(zpre - zb);
+    double mi = 0.0;
     if (melt_on && zb != d.nodata) {
       h0v = max0(z1 - zb);
       hpv = max0(zpre - zb);  // the dilution's hp (common.cpp:216)
@@ -1638,8 +1622,16 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       bmelt += (z1 - zm) * d.arbase;
       h0v = max0(z1 - zb);
     }
+  }
+  __syncthreads();
+  stage_free();
+
+  // ---- Loop 3, Loop 4, friction, store, next Courant ------------------------
+  if (own) {
+    const long long gi = fx_ix(d, irow, icol);
+    const int S0 = tid - BX;  // the south neighbour's north faces
     // Loop 1 wet time (:69-70)
-    if (!(cl & C_DRY)) d.twet[gi] += c.twet_inc;  // dtl / 3600
+    if (!(cl & C_DRY)) d.twet[gi] = tw + c.twet_inc;  // dtl / 3600
 
     // Loop 3 (:93-120)
     double dh = 0.0, dqx = 0.0, dqy = 0.0, qxfP = 0.0, qyfP = 0.0;
@@ -1650,34 +1642,27 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
       qxfP = o[0] * dtl;
       qyfP = o[3] * dtl;
     }
-    if (!wall) {
-      // water leaving the domain this step: through the outflow faces, and
-      // into wall cells (which never take it up, hydrodynamics_calc.cpp:111-117)
-      const unsigned char clE = S.cls[sidx(sr + 1, sc)], clN = S.cls[sidx(sr, sc + 1)];
-      if (irow == d.nr || (clE & C_WALL)) bout += o[0] * d.dxy * dtl;
-      if (icol == d.nc || (clN & C_WALL)) bout += o[3] * d.dxy * dtl;
-    }
+    if (!wall && outE) bout += o[0] * d.dxy * dtl;
+    if (!wall && outN) bout += o[3] * d.dxy * dtl;
     const double qxfW = w[0] * dtl, qyfS = S.f[0][S0] * dtl;
 
     // Loop 4 (:123-154)
     const double z = z1 + dh;
     const double h = max0(z - zb);
-    double qx, qy;
     uint8_t ld;
     if (h < d.hdry || wall) {
       qx = 0.0;
       qy = 0.0;
       ld = 1;
     } else {
-      qx = S.qx[sP] + dqx;
-      qy = S.qy[sP] + dqy;
+      qx += dqx;
+      qy += dqy;
       qx = .1 * qxfW + .8 * qx + .1 * qxfP;
       qy = .1 * qyfS + .8 * qy + .1 * qyfP;
       ld = 0;
     }
     // Extension: semi-implicit Manning friction (n = 0 leaves q unchanged).
     if (d.manning && ld == 0 && !wall) {
-      const double n = d.manning[gi];
       if (n != 0.0) {
         const double qm = sqrt(qx * qx + qy * qy);
         const double h73 = h * h * fx_cbrt(h);
@@ -1706,11 +1691,9 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
     // fe_1 and fn_1 of every cell go to this step's slot, kept ones too
     put_rec64(d, scur + gi, h0v, h, hpv, o[0], o[3], fl1);
     c_h = h;
-    c_qx = qx;
-    c_qy = qy;
   }
   double dtc, hm;
-  courant_cell(d, c_h, c_qx, c_qy, dtc, hm);
+  courant_cell(d, c_h, qx, qy, dtc, hm);
   acc.add(dtc, hm, bmelt, bout);
   return true;
 }
@@ -1724,12 +1707,13 @@ __device__ __forceinline__ void idle_tile(const fx_dev& d, const StepCtl& c, con
 }
 // One tile's step. STAGED: its stencil is in the stage at `stg`, else it is
 // read from global memory. `bad`: this thread's wait for the stage gave up.
-template <bool P32, int BY, bool STAGED>
+// stage_free() is called when no thread reads the stage any more.
+template <bool P32, int BY, bool STAGED, class F>
 __device__ __forceinline__ bool hydro_tile(const fx_dev& d, const StepCtl& c, const fx_tile& tile,
                                            HydroSmem<P32, BY, STAGED>& S, TilePart& acc, const unsigned char* stg,
-                                           int bad) {
-  if constexpr (P32) return hydro_tile32<BY, STAGED>(d, c, tile, S, acc, stg, bad);
-  else return hydro_tile64<BY, STAGED>(d, c, tile, S, acc, stg, bad);
+                                           int bad, F stage_free) {
+  if constexpr (P32) return hydro_tile32<BY, STAGED>(d, c, tile, S, acc, stg, bad, stage_free);
+  else return hydro_tile64<BY, STAGED>(d, c, tile, S, acc, stg, bad, stage_free);
 }
 
 template <bool P32, int BY>
@@ -1743,7 +1727,7 @@ __device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile
   if (!c.live) return;
   TilePart acc = tile_part();
   if (!c.active) idle_tile<P32, BY>(d, c, tile, acc);
-  else hydro_tile<P32, BY, false>(d, c, tile, S, acc, nullptr, 0);
+  else hydro_tile<P32, BY, false>(d, c, tile, S, acc, nullptr, 0, [] {});
   reduce_part(d, S, acc);
 }
 
@@ -1884,7 +1868,8 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (blockIdx.x < ntiles) stage_issue<P32, BY>(d, tm, blockIdx.x, ntx, c.steps - 1, stage0, &bar[0]);
+    for (int q = 0, t = blockIdx.x; q < 2 && t < ntiles; ++q, t += gridDim.x)
+      stage_issue<P32, BY>(d, tm, t, ntx, c.steps - 1, stage0 + q * L::BYTES, &bar[q]);
   }
   __syncthreads();
   unsigned parity = 0u;  // bit q: phase of stage q's barrier
@@ -1895,9 +1880,6 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
   int bx = blockIdx.x % ntx, by = blockIdx.x / ntx;
   const int dbx = gridDim.x % ntx, dby = gridDim.x / ntx;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const int tn = t + gridDim.x;
-    if (tid == 0 && tn < ntiles)
-      stage_issue<P32, BY>(d, tm, tn, ntx, c.steps - 1, stage0 + (st ^ 1) * L::BYTES, &bar[st ^ 1]);
     // wait for this tile's stencil, bounded; each thread waits for itself,
     // and the tile's first barrier (after the stencil is read) tells the
     // whole block whether any wait gave up
@@ -1917,19 +1899,23 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
       bx -= ntx;
       ++by;
     }
-    if (!hydro_tile<P32, BY, true>(d, c, tile, S, acc, stage0 + st * L::BYTES, bad)) {
+    unsigned char* stg = stage0 + st * L::BYTES;
+    const auto next = [&] {  // the stage is free: the tile after next
+      const int tn = t + 2 * gridDim.x;
+      if (tid == 0 && tn < ntiles) stage_issue<P32, BY>(d, tm, tn, ntx, c.steps - 1, stg, &bar[st]);
+    };
+    if (!hydro_tile<P32, BY, true>(d, c, tile, S, acc, stg, bad, next)) {
       // every thread of the block takes this branch
       if (tid == 0) {
         atomicCAS(&d.ctl->error, 0, FX_DEVERR_WAIT_TIMEOUT);
         // let the copy of the next tile, if one was issued, land before the block exits
         long long w = 0;
-        if (tn < ntiles)
+        if (t + gridDim.x < ntiles)
           while (!mbar_try_wait(&bar[st ^ 1], (parity >> (st ^ 1)) & 1u) && ++w < STAGE_SPIN_LIMIT) {
           }
       }
       return;
     }
-    __syncthreads();  // the stage is free for the load issued two tiles later
     st ^= 1;
   }
   reduce_part(d, S, acc);
@@ -2045,7 +2031,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
       const fx_tile tile{0, tl.bx, tl.by, 0};
       // a domain that runs the solver this step was staged (batch_stage)
       if (!c.active) idle_tile<P32, BY>(sd, c, tile, acc);
-      else hydro_tile<P32, BY, true>(sd, c, tile, S, acc, stage0 + st * L::BYTES, 0);
+      else hydro_tile<P32, BY, true>(sd, c, tile, S, acc, stage0 + st * L::BYTES, 0, [] {});
     }
     __syncthreads();  // the stage is free for the copy issued next iteration
     st ^= 1;
