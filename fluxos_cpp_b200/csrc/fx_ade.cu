@@ -43,6 +43,7 @@
 
 #include "fx_common.cuh"
 #include "fx_internal.h"
+#include "fx_unit_order.h"
 
 namespace fxade {
 
@@ -836,8 +837,13 @@ __device__ __forceinline__ bool ade_unit(const fx_dev& d, Ring<T>& R, int jj, in
   }
 }
 
-// One domain: the descriptor is a kernel parameter. Unit u is strip
-// u % nstrips of solute (u / nstrips) % nchem at step u / (nstrips * nchem).
+// The warp's next unit of the launch.
+__device__ __forceinline__ int next_unit(int* counter, int lane) {
+  int u = 0;
+  if (lane == 0) u = atomicAdd(counter, 1);
+  return __shfl_sync(0xffffffffu, u, 0);
+}
+
 // Resident blocks per SM the sweep kernels are compiled for (3: 168
 // registers in FP64, 152 in FP32). More resident warps do not pay: their
 // rings take shared memory from L1, which serves the lanes' skewed reads
@@ -855,24 +861,28 @@ struct AdeBlocks<float> {
   static constexpr int value = FX_ADE_F32_BLOCKS;
 };
 
+// One domain: the descriptor is a kernel parameter. Unit u is solute
+// u % nchem of the step and strip that fx_unit_at gives for u / nchem.
 template <class T>
 __global__ void __launch_bounds__(WARPS * 32, AdeBlocks<T>::value) k_ade_one(const __grid_constant__ fx_dev d,
-                                                                           int nunits) {
+                                                                           int steps) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   Ring<T>& R = reinterpret_cast<Ring<T>*>(smem_raw)[wib];
-  const int nwarps = gridDim.x * WARPS;
   if (!d.ade) return;
-  const int nstrips = (d.nr + ROWS - 1) / ROWS;
-  for (int u = blockIdx.x * WARPS + wib; u < nunits; u += nwarps) {
-    const int s = u % nstrips, k = (u / nstrips) % d.nchem, jj = u / (nstrips * d.nchem);
-    if (!ade_unit<T>(d, R, jj, k, s, lane)) return;
+  const int nstrips = (d.nr + ROWS - 1) / ROWS, nunits = steps * d.nchem * nstrips;
+  fx_unit_walk walk{0, 0};
+  for (int u; (u = next_unit(&d.ctl->ade_next, lane)) < nunits;) {
+    int jj, s;
+    fx_unit_at(u / d.nchem, steps, nstrips, walk, jj, s);
+    if (!ade_unit<T>(d, R, jj, u % d.nchem, s, lane)) return;
   }
 }
 
 // A batch of domains: units come from the unit table; each warp copies its
-// unit's descriptor to its own shared-memory slot.
+// unit's descriptor to its own shared-memory slot. The first domain's control
+// block holds the unit counter.
 template <class T>
 __global__ void __launch_bounds__(WARPS * 32, AdeBlocks<T>::value) k_ade_batch(const fx_dev* __restrict__ devs,
                                                          const fx_unit* __restrict__ units, int nunits) {
@@ -881,9 +891,8 @@ __global__ void __launch_bounds__(WARPS * 32, AdeBlocks<T>::value) k_ade_batch(c
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   Ring<T>& R = reinterpret_cast<Ring<T>*>(smem_raw)[wib];
-  const int nwarps = gridDim.x * WARPS;
   int have = -1;
-  for (int u = blockIdx.x * WARPS + wib; u < nunits; u += nwarps) {
+  for (int u; (u = next_unit(&devs[0].ctl->ade_next, lane)) < nunits;) {
     const fx_unit un = units[u];
     if (un.dom != have) {
       __syncwarp();
@@ -906,21 +915,28 @@ static size_t ade_smem(bool prec32) {
   return (prec32 ? sizeof(fxade::Ring<float>) : sizeof(fxade::Ring<double>)) * fxade::WARPS;
 }
 
-// Units of a domain's launch that are at work at the same time when only
-// their dependencies hold them back: their warp steps over the warp steps of
-// the launch (a strip follows its west strip by about 37 of them, a step the
-// step before by about 48).
+// Warp steps after the start of a launch until unit (jj, s) can start, when only
+// its dependencies hold it back: a strip follows its west strip by about 37, a
+// step the step before by about 48; and until the last unit ends.
+double fx_ade_start(int jj, int s) { return 48.0 * jj + 37.0 * s; }
+double fx_ade_span(int nr, int nc, int steps) {
+  return fx_ade_start(steps, (nr + fxade::ROWS - 1) / fxade::ROWS) + nc;
+}
+// Units of a domain's launch that are then at work at the same time: their
+// warp steps over the warp steps of the launch.
 double fx_ade_active(int nr, int nc, int nchem, int steps) {
   const double strips = (nr + fxade::ROWS - 1) / fxade::ROWS, tw = nc + fxade::ROWS - 1;
-  return steps * nchem * strips * tw / (37.0 * strips + 48.0 * steps + nc);
+  return steps * nchem * strips * tw / fx_ade_span(nr, nc, steps);
 }
 // Which kernel. The chain kernel (a block per unit) takes a unit through its
 // warp steps 3 to 5 times faster but holds 2 (FP64) or 3 (FP32) units per SM
-// against 12, so it wins until the units at work are about its own: 1.8x (FP32)
-// and 2.5x (FP64) at 0.65 units per SM (400^2, 63 steps), 1.5x and 1.7x at 1.6
-// (2048^2, 8 steps), 1.13x and 1.04x at 3.2 (4096^2, 8 steps), 0.97x and
-// 0.92x at 3.5 (2048^2, 20 steps), 0.93x and 0.6x at 6 (1024^2, three solutes).
-bool fx_ade_use_chain(const fx_ade_caps& caps, double active) { return active <= 3.25 * caps.sms; }
+// against 12, so it wins until the units at work are a few times its own. Its
+// gain over the sweep kernel at so many units per SM: FP64 2.3x at 0.65 (400^2,
+// 63 steps), 2.1x at 1.6 (2048^2, 8), 1.28x at 3.2 (4096^2, 8), 1.17x at 3.5
+// (2048^2, 20), 1.04x at 5.1 (1500^2, 63), 0.75x at 6.1 (1024^2, 3 solutes,
+// 31); FP32 1.7x at 0.65, 1.45x at 1.6, 1.27x at 3.2, 1.18x at 6.1, 0.93x at
+// 8 (2048^2, 63), 0.84x at 11 (4096^2, 31).
+bool fx_ade_use_chain(const fx_ade_caps& caps, double active) { return active <= caps.chain_active; }
 
 void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const fx_ade_caps& caps, bool chain, bool prec32,
                    cudaStream_t s) {
@@ -935,12 +951,12 @@ void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const f
 void fx_launch_ade_one(const fx_dev& d, int steps, const fx_ade_caps& caps, cudaStream_t s) {
   const int nunits = steps * d.nchem * ((d.nr + fxade::ROWS - 1) / fxade::ROWS);
   if (fx_ade_use_chain(caps, fx_ade_active(d.nr, d.nc, d.nchem, steps))) {
-    fx_chain_launch_one(d, nunits, caps.chain, s);
+    fx_chain_launch_one(d, steps, caps.chain, s);
     return;
   }
   const int nblocks = std::max(1, std::min((nunits + fxade::WARPS - 1) / fxade::WARPS, caps.sweep));
-  if (d.prec32) fxade::k_ade_one<float><<<nblocks, fxade::WARPS * 32, ade_smem(true), s>>>(d, nunits);
-  else fxade::k_ade_one<double><<<nblocks, fxade::WARPS * 32, ade_smem(false), s>>>(d, nunits);
+  if (d.prec32) fxade::k_ade_one<float><<<nblocks, fxade::WARPS * 32, ade_smem(true), s>>>(d, steps);
+  else fxade::k_ade_one<double><<<nblocks, fxade::WARPS * 32, ade_smem(false), s>>>(d, steps);
 }
 
 // Appends the ADE units of domain `dom` for a batch of `steps` steps, in the
@@ -1002,7 +1018,7 @@ int fx_ade_caps_for(bool prec32, fx_ade_caps* out) {
         max_blocks_of(fxade::k_ade_batch<double>, ade_smem(false), nsm, &b))
       return -1;
   }
-  out->sms = nsm;
+  out->chain_active = (prec32 ? 7.0 : 4.25) * nsm;
   out->sweep = std::min(a, b);
   return out->sweep > 0 ? fx_chain_blocks(prec32, &out->chain) : -1;
 }

@@ -37,7 +37,8 @@
 // rounds behind on the same and the next strip, and add_meteo's dilution
 // (common.cpp:226-234) is applied to each record as it is formed.
 //
-// Units are handed out in dependency order by a counter (fx_ctl::ade_next),
+// Units are handed out by a counter (fx_ctl::ade_next) in an order that has
+// every unit behind the ones it waits for (fx_unit_order.h, fx_batch.cu),
 // so whichever blocks are resident hold the oldest unfinished units and
 // never wait on a unit that no block has taken. Strips of one step hand over
 // through a small boundary buffer (per column: updated c, pfe, re-scaled c
@@ -52,6 +53,7 @@
 
 #include "fx_common.cuh"
 #include "fx_internal.h"
+#include "fx_unit_order.h"
 
 namespace fxchain {
 
@@ -118,6 +120,8 @@ struct Smem {
   int c_taken;  // rounds of concentrations the face warps have read
   int abort;    // a wait gave up
   int unit;
+  int jj, k, s;  // the one-domain form: the unit's step, solute and strip
+  fx_unit_walk walk;
 };
 
 // The state fields of the sweep in precision T.
@@ -1096,13 +1100,15 @@ __device__ __forceinline__ void init_smem(Smem<T>& M) {
 
 // Takes the block's next unit (every thread calls it); -1 when there is none
 // or a wait gave up.
-template <class T>
-__device__ __forceinline__ int next_unit(Smem<T>& M, int* counter, int nunits) {
+// `decode` is called with it by the thread that took it.
+template <class T, class F>
+__device__ __forceinline__ int next_unit(Smem<T>& M, int* counter, int nunits, F decode) {
   __syncthreads();  // every warp is done with the last unit
   if (threadIdx.x == 0) {
     const int u = atomicAdd(counter, 1);
     M.unit = (u < nunits && !M.abort) ? u : -1;
     M.done = M.c_taken = 0;
+    if (M.unit >= 0) decode(M.unit);
   }
   // what the first warp step finds to its west and south: the ghost cells
   if (threadIdx.x < RS) M.bh[RECS - 1][threadIdx.x][0] = M.bh[RECS - 1][threadIdx.x][1] = T(0);
@@ -1120,20 +1126,24 @@ struct ChainBlocks {
   static constexpr int value = sizeof(T) == 8 ? 2 : 3;
 };
 
-// One domain: the descriptor is a kernel parameter. Unit u is strip
-// u % nstrips of solute (u / nstrips) % nchem at step u / (nstrips * nchem).
+// One domain: the descriptor is a kernel parameter. Unit u is solute
+// u % nchem of the step and strip that fx_unit_at gives for u / nchem.
 template <class T>
-__global__ void __launch_bounds__(NTHREADS, ChainBlocks<T>::value) k_chain_one(const __grid_constant__ fx_dev d, int nunits) {
+__global__ void __launch_bounds__(NTHREADS, ChainBlocks<T>::value) k_chain_one(const __grid_constant__ fx_dev d, int steps) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem<T>& M = *reinterpret_cast<Smem<T>*>(smem_raw);
   if (!d.ade) return;
   init_smem(M);
   const int nstrips = (d.nr + ROWS - 1) / ROWS;
+  if (threadIdx.x == 0) M.walk = fx_unit_walk{0, 0};
   int c_round = 0, k_round = 0, b_round = 0;
   for (;;) {
-    const int u = next_unit(M, &d.ctl->ade_next, nunits);
+    const int u = next_unit(M, &d.ctl->ade_next, steps * d.nchem * nstrips, [&](int i) {
+      M.k = i % d.nchem;
+      fx_unit_at(i / d.nchem, steps, nstrips, M.walk, M.jj, M.s);
+    });
     if (u < 0) break;
-    run_unit<T>(d, M, u / (nstrips * d.nchem), (u / nstrips) % d.nchem, u % nstrips, c_round, k_round, b_round);
+    run_unit<T>(d, M, M.jj, M.k, M.s, c_round, k_round, b_round);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -1151,7 +1161,7 @@ __global__ void __launch_bounds__(NTHREADS, ChainBlocks<T>::value) k_chain_batch
   int have = -1, c_round = 0, k_round = 0, b_round = 0;
   int* counter = &devs[0].ctl->ade_next;
   for (;;) {
-    const int u = next_unit(M, counter, nunits);
+    const int u = next_unit(M, counter, nunits, [](int) {});
     if (u < 0) break;
     const fx_unit un = units[u];
     if (un.dom != have) {
@@ -1178,10 +1188,11 @@ void fx_chain_launch(const fx_dev* devs, const fx_unit* units, int nunits, int m
   if (prec32) fxchain::k_chain_batch<float><<<nblocks, fxchain::NTHREADS, chain_smem(true), s>>>(devs, units, nunits);
   else fxchain::k_chain_batch<double><<<nblocks, fxchain::NTHREADS, chain_smem(false), s>>>(devs, units, nunits);
 }
-void fx_chain_launch_one(const fx_dev& d, int nunits, int max_blocks, cudaStream_t s) {
+void fx_chain_launch_one(const fx_dev& d, int steps, int max_blocks, cudaStream_t s) {
+  const int nunits = steps * d.nchem * ((d.nr + fxchain::ROWS - 1) / fxchain::ROWS);
   const int nblocks = std::max(1, std::min(nunits, max_blocks));
-  if (d.prec32) fxchain::k_chain_one<float><<<nblocks, fxchain::NTHREADS, chain_smem(true), s>>>(d, nunits);
-  else fxchain::k_chain_one<double><<<nblocks, fxchain::NTHREADS, chain_smem(false), s>>>(d, nunits);
+  if (d.prec32) fxchain::k_chain_one<float><<<nblocks, fxchain::NTHREADS, chain_smem(true), s>>>(d, steps);
+  else fxchain::k_chain_one<double><<<nblocks, fxchain::NTHREADS, chain_smem(false), s>>>(d, steps);
 }
 
 // Resident blocks of a kernel, after raising its dynamic shared memory limit.

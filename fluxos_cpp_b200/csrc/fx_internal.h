@@ -13,7 +13,7 @@
 // per unit (fx_ade.cu) and the one of a block per unit (fx_ade_chain.cu).
 struct fx_ade_caps {
   int sweep = 0, chain = 0;
-  int sms = 0;  // SMs of the device
+  double chain_active = 0;  // the most units at work that the chain kernel takes (fx_ade_use_chain)
 };
 
 struct fx_ctx {
@@ -88,6 +88,8 @@ void fx_launch_courant_scan(const fx_dev* devs, const fx_tile* tiles, int ntiles
 // chain: which of the two kernels (fx_ade_use_chain of the sum of the domains'
 // fx_ade_active). fx_launch_ade_one picks its own for the given steps.
 double fx_ade_active(int nr, int nc, int nchem, int steps);
+double fx_ade_start(int jj, int s);
+double fx_ade_span(int nr, int nc, int steps);
 bool fx_ade_use_chain(const fx_ade_caps& caps, double active);
 void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const fx_ade_caps& caps, bool chain, bool prec32,
                    cudaStream_t s);
@@ -110,5 +112,5 @@ int fx_ade_rows_per_strip();
 int fx_ade_caps_for(bool prec32, fx_ade_caps* out);
 // The ADE kernel with a block per unit (fx_ade_chain.cu).
 void fx_chain_launch(const fx_dev* devs, const fx_unit* units, int nunits, int max_blocks, bool prec32, cudaStream_t s);
-void fx_chain_launch_one(const fx_dev& d, int nunits, int max_blocks, cudaStream_t s);
+void fx_chain_launch_one(const fx_dev& d, int steps, int max_blocks, cudaStream_t s);
 int fx_chain_blocks(bool prec32, int* out);
