@@ -45,10 +45,5 @@ __device__ __forceinline__ double over(double a, double b, double y) {
   if ((e >= (1400u << 20)) & !zero) q = plain_div(a, b);
   return q;
 }
-// One quotient, by a division that skips a numerator of 0 over an ordinary b.
-__device__ __forceinline__ double zdiv(double a, double b) {
-  const unsigned e = (unsigned)(__double2hiint(b) & 0x7ff00000);
-  return (a == 0.0) & (e != 0u) & (e != 0x7ff00000u) ? a * b : plain_div(a, b);
-}
 
 }  // namespace fx

@@ -1931,17 +1931,12 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
 // memory while the block works on its tiles, and the block's Courant and
 // budget partials go to a domain when the block leaves it.
 
-// Thread 0: stage tile t of the table into `stg` if its domain runs the
-// solver this step; returns whether a copy was issued.
+// Thread 0: stage tile `tl` into `stg` if its domain runs the solver this step;
+// returns whether a copy was issued.
 template <bool P32, int BY>
-__device__ __forceinline__ bool batch_stage(const fx_dev* __restrict__ devs, const fx_tmaps* __restrict__ tms,
-                                            const fx_tile* __restrict__ tiles, int t, unsigned char* stg,
-                                            unsigned long long* bar, int& fenced) {
-  const fx_tile tl = tiles[t];
-  const fx_dev& dm = devs[tl.dom];
-  const fx_ctl& g = *dm.ctl;
-  if (!g.live || !g.active) return false;
-  const fx_tmaps& tm = tms[tl.dom];
+__device__ __forceinline__ bool batch_stage(const fx_dev& d, bool runs, long long step_prev, const fx_tmaps& tm,
+                                            const fx_tile& tl, unsigned char* stg, unsigned long long* bar, int& fenced) {
+  if (!runs) return false;
   if (fenced != tl.dom) {
     // the maps were written by a host copy before the launch; order the
     // tensor-map proxy's reads of a domain's maps after it, once per domain
@@ -1949,8 +1944,8 @@ __device__ __forceinline__ bool batch_stage(const fx_dev* __restrict__ devs, con
       asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&tm.m[f]) : "memory");
     fenced = tl.dom;
   }
-  const int ntx = (dm.nr + TX - 1) / TX;
-  stage_issue<P32, BY>(dm, tm, tl.by * ntx + tl.bx, ntx, g.steps - 1, stg, bar);
+  const int ntx = (d.nr + TX - 1) / TX;
+  stage_issue<P32, BY>(d, tm, tl.by * ntx + tl.bx, ntx, step_prev, stg, bar);
   return true;
 }
 
@@ -1963,8 +1958,8 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
   __shared__ fx_dev sd;
   __shared__ StepCtl sc;
   __shared__ __align__(8) unsigned long long bar[2];
-  __shared__ int staged[2];  // the tile each stage holds (-1: none)
-  __shared__ int abort_flag;
+  __shared__ int staged[2];      // the tile each stage holds (-1: none)
+  __shared__ fx_tile entry[4];   // the table's entries of the tiles under way
   extern __shared__ __align__(128) unsigned char dyn[];
   unsigned char* stage0 = dyn + ((128 - (smem_u32(dyn) & 127)) & 127);
   const int tid = threadIdx.y * BX + threadIdx.x;
@@ -1972,20 +1967,39 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
   const int t1 = (int)((long long)ntiles * (blockIdx.x + 1) / gridDim.x);
   if (t0 >= t1) return;
   int fenced = -1;  // thread 0: the domain whose maps it last fenced
+  // Thread 0: stage tile t, whose entry is `tl`, into stage q. The descriptor
+  // and control block of the domain at hand are in shared memory; another
+  // domain's are read from global memory, once per domain and block.
+  const auto stage = [&](int t, const fx_tile& tl, int q, int at_hand) {
+    entry[t & 3] = tl;
+    bool on;
+    if (tl.dom == at_hand) {
+      on = batch_stage<P32, BY>(sd, sc.live && sc.active, sc.steps - 1, tms[tl.dom], tl, stage0 + q * L::BYTES, &bar[q],
+                                fenced);
+    } else {
+      const fx_dev& d = devs[tl.dom];
+      const fx_ctl& g = *d.ctl;
+      on = batch_stage<P32, BY>(d, g.live && g.active, g.steps - 1, tms[tl.dom], tl, stage0 + q * L::BYTES, &bar[q],
+                                fenced);
+    }
+    staged[q] = on ? t : -1;
+  };
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    abort_flag = 0;
-    staged[0] = batch_stage<P32, BY>(devs, tms, tiles, t0, stage0, &bar[0], fenced) ? t0 : -1;
     staged[1] = -1;
+    stage(t0, tiles[t0], 0, -1);
+    if (t0 + 1 < t1) stage(t0 + 1, tiles[t0 + 1], 1, -1);
   }
   __syncthreads();
   unsigned parity = 0u;  // bit q: phase of stage q's barrier
   int st = 0, dom = -1;
   TilePart acc = tile_part();
   for (int t = t0; t < t1; ++t) {
-    const fx_tile tl = tiles[t];
+    const fx_tile tl = entry[t & 3];
+    fx_tile after{};  // thread 0: the entry of the tile after next, loaded ahead of its use
+    if (tid == 0 && t + 2 < t1) after = tiles[t + 2];
     if (tl.dom != dom) {
       if (dom >= 0) reduce_part(sd, S, acc);  // the partials of the domain the block leaves
       acc = tile_part();
@@ -1994,46 +2008,47 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
       unsigned long long* dst = reinterpret_cast<unsigned long long*>(&sd);
       for (int i = tid; i < (int)(sizeof(fx_dev) / 8); i += BX * BY) dst[i] = src[i];
       __syncthreads();
-      if (tid == 0) {
-        read_ctl(sd, sc);
-      }
+      if (tid == 0) read_ctl(sd, sc);
       __syncthreads();
       dom = tl.dom;
     }
-    if (tid == 0)
-      staged[st ^ 1] = (t + 1 < t1 && batch_stage<P32, BY>(devs, tms, tiles, t + 1, stage0 + (st ^ 1) * L::BYTES,
-                                                           &bar[st ^ 1], fenced))
-                           ? t + 1 : -1;
     const bool mine = staged[st] == t;  // this tile's stencil is (being) staged
+    int bad = 0;
     if (mine) {
       long long it = 0;
       while (!mbar_try_wait(&bar[st], (parity >> st) & 1u)) {
         if (++it > STAGE_SPIN_LIMIT) {
-          abort_flag = 1;
+          bad = 1;
           break;
         }
       }
       parity ^= 1u << st;
     }
-    __syncthreads();
-    if (abort_flag) {
+    const auto next = [&] {  // the stage is free: the tile after next
       if (tid == 0) {
-        atomicCAS(&sd.ctl->error, 0, FX_DEVERR_WAIT_TIMEOUT);
-        long long w = 0;  // let a copy already issued for the next tile land before the block exits
-        if (staged[st ^ 1] >= 0)
-          while (!mbar_try_wait(&bar[st ^ 1], (parity >> (st ^ 1)) & 1u) && ++w < STAGE_SPIN_LIMIT) {
-          }
+        if (t + 2 < t1) stage(t + 2, after, st, dom);
+        else staged[st] = -1;
       }
-      return;
-    }
+    };
     const StepCtl c = sc;
-    if (c.live) {
-      const fx_tile tile{0, tl.bx, tl.by, 0};
-      // a domain that runs the solver this step was staged (batch_stage)
-      if (!c.active) idle_tile<P32, BY>(sd, c, tile, acc);
-      else hydro_tile<P32, BY, true>(sd, c, tile, S, acc, stage0 + st * L::BYTES, 0, [] {});
+    const fx_tile tile{0, tl.bx, tl.by, 0};
+    if (c.live && c.active) {  // such a domain's tiles are staged
+      if (!hydro_tile<P32, BY, true>(sd, c, tile, S, acc, stage0 + st * L::BYTES, bad, next)) {
+        // every thread of the block takes this branch
+        if (tid == 0) {
+          atomicCAS(&sd.ctl->error, 0, FX_DEVERR_WAIT_TIMEOUT);
+          long long w = 0;  // let a copy already issued for the next tile land before the block exits
+          if (staged[st ^ 1] >= 0)
+            while (!mbar_try_wait(&bar[st ^ 1], (parity >> (st ^ 1)) & 1u) && ++w < STAGE_SPIN_LIMIT) {
+            }
+        }
+        return;
+      }
+    } else {
+      if (c.live) idle_tile<P32, BY>(sd, c, tile, acc);
+      next();
+      __syncthreads();  // what next() wrote is read two tiles on, with no barrier between when the next is idle too
     }
-    __syncthreads();  // the stage is free for the copy issued next iteration
     st ^= 1;
   }
   if (dom >= 0) reduce_part(sd, S, acc);
