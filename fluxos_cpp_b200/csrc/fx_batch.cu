@@ -39,6 +39,7 @@ struct fx_batch {
   bool hydro_tma = false;  // the current graph uses it
   int tma_blocks = 0;
   int tile_rows = 8;              // hydrodynamic tile shape of the batch's launches
+  bool rows_set = false;          // chosen by the user or the autotuner, not fx_default_tile_rows
   int k_limit = FX_MAX_SLOTS;     // upper bound on steps per graph (ADE sweeps in flight)
   bool dirty = true;  // membership or a descriptor changed: rebuild tables and graph
   cudaGraphExec_t graph = nullptr;
@@ -77,6 +78,14 @@ static int rebuild(fx_batch* b) {
   b->K = b->k_limit;
   for (fx_ctx* c : b->doms) b->K = std::min(b->K, c->batch_steps);
   if (n == 0) b->K = 1;
+  if (!b->rows_set) {
+    std::vector<int> nr, nc;
+    for (fx_ctx* c : b->doms) {
+      nr.push_back(c->g.nrows);
+      nc.push_back(c->g.ncols);
+    }
+    b->tile_rows = fx_default_tile_rows(n > 0 && b->doms[0]->d.prec32 != 0, nr, nc);
+  }
   std::vector<fx_dev> devs(n);
   std::vector<fx_tile> tiles;
   std::vector<fx_unit> units;
@@ -280,6 +289,7 @@ int fx_batch_set_option(fx_batch* b, const char* name, long long v) {
   if (!strcmp(name, "tile_rows")) {
     if (!fx_tile_rows_ok((int)v)) return fx_fail(nullptr, FX_ERR_ARG, "tile_rows must be 4, 8 or 16");
     b->tile_rows = (int)v;
+    b->rows_set = true;
   } else if (!strcmp(name, "steps_in_flight")) {
     if (v < 1 || v > FX_MAX_SLOTS - 1) return fx_fail(nullptr, FX_ERR_ARG, "steps_in_flight must be 1..63");
     b->k_limit = (int)v;
@@ -351,10 +361,11 @@ int fx_batch_autotune(fx_batch* b, int trial_steps, int* tile_rows, int* steps_i
   };
   int best_rows = b->tile_rows;
   const int rows[3] = {4, 8, 16};
-  rc = sweep(rows, 3, [&](int r) { b->tile_rows = r; b->dirty = true; }, [&](int) { return trial_steps; },
+  rc = sweep(rows, 3, [&](int r) { b->tile_rows = r; b->rows_set = true; b->dirty = true; }, [&](int) { return trial_steps; },
              &best_rows);
   if (rc) return rc;
   b->tile_rows = best_rows;
+  b->rows_set = true;
   b->dirty = true;
   int best_k = std::min(b->k_limit, kmax);
   int ks[6], nk = 0;

@@ -382,7 +382,7 @@ int fx_create(const fx_grid* g, const fx_params* p, fx_ctx** out) {
     fx_tiles_of(0, g->nrows, g->ncols, 4, tiles);
     if ((rc = dev_alloc(c, (void**)&c->d_tiles, sizeof(fx_tile) * tiles.size())) != FX_OK) goto fail;
     if ((rc = dev_alloc(c, (void**)&c->d_dev, sizeof(fx_dev))) != FX_OK) goto fail;
-    if ((rc = set_tile_rows(c, 8)) != FX_OK) goto fail;
+    if ((rc = set_tile_rows(c, fx_default_tile_rows(d.prec32 != 0, {g->nrows}, {g->ncols}))) != FX_OK) goto fail;
   }
   e = cudaMallocHost((void**)&c->ctl_host, sizeof(fx_ctl));
   if (e != cudaSuccess) {

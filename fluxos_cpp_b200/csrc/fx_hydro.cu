@@ -2314,6 +2314,36 @@ void launch_hydro_one(const fx_dev& d, cudaStream_t s) {
 
 bool fx_tile_rows_ok(int r) { return r == 4 || r == 8 || r == 16; }
 
+static long long tiles_of(int nr, int nc, int rows) {
+  return (long long)((nr + fx::TX - 1) / fx::TX) * ((nc + rows - 2) / (rows - 1));
+}
+// The tile shape where none is set, for domains of nr[i] x nc[i] cells.
+// * 4 rows while all such tiles are resident at once (5 blocks an SM): a step
+//   is then one tile's latency, and the smallest tile's is the shortest
+//   (200 x 200 cells FP64 16.3 us against 18.0 with 8 rows, FP32 13.3 against
+//   13.8; 257 x 257 FP64, one tile in 20 too many, 22.1 against 20.3).
+// * 16 rows in FP32 when every block has ten such tiles or more: fewer halo
+//   cells are read and updated (2048 x 2048 cells 0.223 ms against 0.236,
+//   1280 x 1280 96 us against 101, 64 domains of 200 x 200 199 us against 204);
+//   with eight a block (1024 x 1024) it is 2 % less with water everywhere and
+//   5 % more after a dam break. In FP64 they spill (2048 x 2048 0.73 against 0.58 ms).
+// * 8 rows otherwise.
+int fx_default_tile_rows(bool prec32, const std::vector<int>& nr, const std::vector<int>& nc) {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 8;
+  long long small = 0, large = 0;
+  bool staged = true;  // boxes of 16 rows fit every domain
+  for (size_t i = 0; i < nr.size(); ++i) {
+    small += tiles_of(nr[i], nc[i], 4);
+    large += tiles_of(nr[i], nc[i], 16);
+    staged &= nc[i] >= 16;
+  }
+  if (small <= 5LL * nsm) return 4;
+  return prec32 && staged && large >= 10LL * fx::min_blocks<true, 16>() * nsm ? 16 : 8;
+}
+
 void fx_launch_hydro(const fx_dev* devs, const fx_tile* tiles, int ntiles, bool prec32, int tile_rows,
                      cudaStream_t s) {
   if (tile_rows == 4) launch_hydro_batch<4>(devs, tiles, ntiles, prec32, s);

@@ -84,6 +84,7 @@ int fx_hydro_batch_tma_blocks(bool prec32, int tile_rows, int* out);
 // Tensor maps of a context's stencil fields for a tile shape (fx_capi.cu).
 int fx_build_tmaps_for(fx_ctx* c, int tile_rows, fx_tmaps* out);
 bool fx_tma_fits(const fx_ctx* c, int tile_rows);
+int fx_default_tile_rows(bool prec32, const std::vector<int>& nr, const std::vector<int>& nc);
 void fx_launch_courant_scan(const fx_dev* devs, const fx_tile* tiles, int ntiles, int tile_rows, cudaStream_t s);
 // chain: which of the two kernels (fx_ade_use_chain of the sum of the domains'
 // fx_ade_active). fx_launch_ade_one picks its own for the given steps.

@@ -141,7 +141,7 @@ int fx_set_melt_field(fx_ctx* ctx, const double* mult_grid);
  * device every step; 0, the default, skips those stores for cells that end a
  * step wet, whose values are never read back by a later step);
  * "tile_rows" (4, 8 or 16: hydrodynamic tiles of 31 x (tile_rows - 1) cells,
- * 32 x tile_rows threads; default 8); "tma" (1, the default: a persistent
+ * 32 x tile_rows threads; by default the size of the grid decides); "tma" (1, the default: a persistent
  * hydrodynamic kernel whose blocks stage each tile's stencil into shared
  * memory by TMA while computing the previous tile; 0: one block per tile
  * loading its stencil itself). Results depend on neither.
