@@ -49,12 +49,26 @@ namespace fxade {
 
 constexpr int ROWS = 30;      // rows per strip (lanes 0..29 compute)
 constexpr int WARPS = 4;      // warps per block
-constexpr int CHUNK = 4;      // steps between progress checks and publications (the lag between
-                              // strips is 2 * CHUNK + ROWS - 1 warp steps)
 constexpr int RING = 4;       // per-lane prefetch slots (a power of two); a deeper ring takes shared
                               // memory from L1, which the lanes' skewed reads depend on (measured:
                               // 8 slots made the FP64 sweep 2.5x slower)
-constexpr int DIST = 2;       // prefetch distance in columns (< RING)
+// CHUNK: steps between progress checks and publications. A publication makes
+// the warp wait for its last writes; the lag between strips is
+// 2 * CHUNK + ROWS - 1 warp steps. DIST: prefetch distance in columns (< RING).
+// FP32 sweeps are many warps wide when they come here (fx_ade_use_chain) and
+// can do with the longer lag: ms a step with 4 and 2, 8 and 3, 16 and 3, at
+// 4096^2 cells, 63 steps 0.545, 0.484, 0.462; 2048^2, 63 steps 0.199, 0.186,
+// 0.196; 1024^2, three solutes 0.178, 0.169, 0.191. FP64, fewer warps of more
+// work, does not gain: 4096^2, 20 steps 1.519 with 4, 1.504 with 8, 1.775 with
+// 16; 2048^2 0.554, 0.580, 0.690.
+template <class T>
+struct Shape {
+  static constexpr int CHUNK = 4, DIST = 2;
+};
+template <>
+struct Shape<float> {
+  static constexpr int CHUNK = 8, DIST = 3;
+};
 constexpr long long SPIN_LIMIT = 1LL << 20;  // polls (well under a second) before giving up
 constexpr long long HOLD_SPIN_LIMIT = 1LL << 12;  // the same with fx_dev.ade_hold (a test of the timeout path)
 
@@ -584,6 +598,7 @@ __device__ __forceinline__ bool wait_deps(const fx_dev& d, Deps& D, int need_w, 
 // Returns false when a wait gave up.
 template <class T>
 __device__ __forceinline__ bool ade_unit(const fx_dev& d, Ring<T>& R, int jj, int k, int s, int lane) {
+  constexpr int CHUNK = Shape<T>::CHUNK, DIST = Shape<T>::DIST;
   {
     const fx_ctl& cc = *d.ctl;
     // this batch's live steps are consecutive: the jj-th is minstep + jj
@@ -934,8 +949,8 @@ double fx_ade_active(int nr, int nc, int nchem, int steps) {
 // gain over the sweep kernel at so many units per SM: FP64 2.3x at 0.65 (400^2,
 // 63 steps), 2.1x at 1.6 (2048^2, 8), 1.28x at 3.2 (4096^2, 8), 1.17x at 3.5
 // (2048^2, 20), 1.04x at 5.1 (1500^2, 63), 0.75x at 6.1 (1024^2, 3 solutes,
-// 31); FP32 1.7x at 0.65, 1.45x at 1.6, 1.27x at 3.2, 1.18x at 6.1, 0.93x at
-// 8 (2048^2, 63), 0.84x at 11 (4096^2, 31).
+// 31); FP32 1.6x at 0.65, 1.4x at 1.6, 1.2x at 3.2, 1.13x at 6.1, 0.85x at 8
+// (2048^2, 63), 0.73x at 11 (4096^2, 31).
 bool fx_ade_use_chain(const fx_ade_caps& caps, double active) { return active <= caps.chain_active; }
 
 void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const fx_ade_caps& caps, bool chain, bool prec32,
