@@ -488,12 +488,19 @@ __global__ void k_rec_put(const __grid_constant__ fx_dev d, R* __restrict__ rec,
         if (k != cur) rec[N * ((long long)k * d.plane + i) + comp] = v;
   }
 }
+// Component `comp` of a field of N values of type R a cell in `planes` planes,
+// of the plane that holds the state after the last step: found on the device,
+// where the host would wait for the control block.
 template <class R, int N>
-__global__ void k_rec_get(const R* __restrict__ rec, int comp, double* __restrict__ dst, long long plane) {
+__global__ void k_current(const R* __restrict__ field, int planes, const fx_ctl* __restrict__ ctl, int comp,
+                          double* __restrict__ dst, long long plane) {
+  const R* src = field + N * (ctl->steps % planes) * plane + comp;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < plane; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = (double)rec[N * i + comp];
+    dst[i] = (double)src[N * i];
 }
 }  // extern "C++"
+// A step budget of n steps from here.
+__global__ void k_set_stop(fx_ctl* ctl, long long n) { ctl->stop_after = ctl->steps + n; }
 // z = zb + (eta + eta_lo) of the FP32 state (the order of get_z32's host sum before).
 __global__ void k_z_of_eta(const double* __restrict__ zb, const float* __restrict__ eta,
                            const float* __restrict__ lo, double* __restrict__ z, long long n) {
@@ -637,29 +644,22 @@ int fx_download(fx_ctx* c, const char* field, double* host) {
     std::fill(host, host + ((size_t)c->d.nr + 2) * ((size_t)c->d.nc + 2), 0.0);
     return FX_OK;
   }
-  if (f.rec >= 0) {  // FP32 per-step field: one component of the current slot's records
-    int rc = read_ctl(c);
-    if (rc) return rc;
-    const long long o = fx_slot(c->d, c->ctl_host->steps);
-    if (c->d.prec32)
-      k_rec_get<float, 8><<<plane_grid(c->d.plane), 256, 0, c->stream>>>(fx_rec(c->d, o), f.rec, c->stage,
-                                                                        c->d.plane);
-    else
-      k_rec_get<double, FX_R64_N><<<plane_grid(c->d.plane), 256, 0, c->stream>>>(fx_rec64(c->d, o), f.rec,
-                                                                                c->stage, c->d.plane);
-    FX_CK(c, cudaGetLastError());
-    if ((rc = copy_out(c, host, c->stage))) return rc;
-    FX_CK(c, cudaStreamSynchronize(c->stream));
-    return FX_OK;
-  }
-  const size_t esz = f.f32 ? sizeof(float) : sizeof(double);
-  const char* src = (const char*)f.ptr;
-  if (f.slot || f.pair) {
-    int rc = read_ctl(c);
-    if (rc) return rc;
-    src += (f.slot ? fx_slot(c->d, c->ctl_host->steps) : fx_pp(c->d, c->ctl_host->steps)) * esz;
-  }
-  return get_grid(c, src, f.f32, host);
+  const int grid = plane_grid(c->d.plane), planes = f.slot || f.rec >= 0 ? c->d.nslot : 2;
+  if (f.rec >= 0 && c->d.prec32)  // a component of the slot records
+    k_current<float, 8><<<grid, 256, 0, c->stream>>>(reinterpret_cast<const float*>(c->d.rec32), planes, c->d.ctl, f.rec,
+                                                     c->stage, c->d.plane);
+  else if (f.rec >= 0)
+    k_current<double, FX_R64_N><<<grid, 256, 0, c->stream>>>(c->d.rec64, planes, c->d.ctl, f.rec, c->stage, c->d.plane);
+  else if ((f.slot || f.pair) && f.f32)
+    k_current<float, 1><<<grid, 256, 0, c->stream>>>((const float*)f.ptr, planes, c->d.ctl, 0, c->stage, c->d.plane);
+  else if (f.slot || f.pair)
+    k_current<double, 1><<<grid, 256, 0, c->stream>>>((const double*)f.ptr, planes, c->d.ctl, 0, c->stage, c->d.plane);
+  else return get_grid(c, f.ptr, f.f32, host);
+  FX_CK(c, cudaGetLastError());
+  const int rc = copy_out(c, host, c->stage);
+  if (rc) return rc;
+  FX_CK(c, cudaStreamSynchronize(c->stream));
+  return FX_OK;
 }
 
 // The flag byte of each grid cell from the two uploaded float planes (1.0 =
@@ -937,13 +937,9 @@ int fx_step(fx_ctx* c, int nsteps, fx_status* st) {
     int rc = fx_prepare(c);
     if (rc) return rc;
   }
-  int rc = read_ctl(c);
-  if (rc) return rc;
-  if (c->ctl_host->error) {  // a kernel gave up a wait: the state is not stepped further
-    fx_fill_status(*c->ctl_host, st);
-    return status_rc(c);
-  }
-  if ((rc = set_stop(c, c->ctl_host->steps + nsteps))) return rc;
+  // with a kernel's error standing, no step of these runs (k_finalize)
+  int rc;
+  k_set_stop<<<1, 1, 0, c->stream>>>(c->d.ctl, nsteps);
   if ((rc = ensure_graph(c))) return rc;
   int left = nsteps;
   while (left >= c->batch_steps) {
