@@ -4,7 +4,7 @@
 // A batch of K steps is one CUDA graph: open the batch in every domain, then
 // K times (clock update of every domain, one hydrodynamic launch over the
 // concatenated tile table of all domains), then one ADE launch over the
-// interleaved unit table of all domains (fx_ade.cu). The hydrodynamic launch
+// unit table of all domains merged by start (fx_ade.cu). The hydrodynamic launch
 // is the persistent TMA-staged batch kernel (each domain's stencil fields
 // staged through its own tensor maps, kept in a device array) when every
 // member's grid is large enough for a staged box; otherwise one block per

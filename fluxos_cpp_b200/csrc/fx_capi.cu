@@ -940,7 +940,10 @@ int fx_step(fx_ctx* c, int nsteps, fx_status* st) {
   // with a kernel's error standing, no step of these runs (k_finalize)
   int rc;
   k_set_stop<<<1, 1, 0, c->stream>>>(c->d.ctl, nsteps);
-  if ((rc = ensure_graph(c))) return rc;
+  // the graph holds a whole batch of steps: fewer are launched one by one, and
+  // a caller that never takes a batch at once does not pay for it (400 us on
+  // the first call)
+  if ((rc = nsteps >= c->batch_steps ? ensure_graph(c) : fx_sync_dev(c))) return rc;
   int left = nsteps;
   while (left >= c->batch_steps) {
     FX_CK(c, cudaGraphLaunch(c->graph_exec, c->stream));

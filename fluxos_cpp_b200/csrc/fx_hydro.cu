@@ -1,17 +1,17 @@
-// FP64 hydrodynamic step of FLUXOS-OVERLAND for sm_100a.
+// Hydrodynamic step of FLUXOS-OVERLAND for sm_100a, FP64 and FP32.
 //
-// One launch of k_hydro performs, for a 32 x 8 tile of cells:
+// One launch of k_hydro_* performs, tile by tile (31 x BY-1 cells):
 //   * the snowmelt forcing of common.cpp:210-262 (add_meteo), including the
 //     solute dilution, applied on the fly to every cell the tile reads;
 //   * Loop 1 of hydrodynamics_calc.cpp:53-73 (depth, wet flag, wet time);
 //   * Loop 2 (:76-90): the east and north face fluxes of solver_wet
 //     (solver_wetdomain.cpp:27-342) and solver_dry (solver_drydomain.cpp:27-194)
-//     for the tile and its west/south halo, each face once, held in shared
-//     memory and used by both cells that share it;
+//     for the tile and its west/south halo, each face once, by one thread,
+//     and used by both cells that share it;
 //   * Loop 3 (:93-120) and Loop 4 (:123-154): divergence and update;
 //   * the optional Manning friction extension;
 //   * the per-cell part of the NEXT step's Courant scan (main.cpp:300-323),
-//     reduced with warp shuffles and one atomic per block.
+//     kept per thread and reduced once per block with one atomic.
 // k_finalize then turns the reduction into the next dt and advances the
 // clock on the device, so a run of steps needs no host round trip.
 //
@@ -1791,10 +1791,10 @@ static_assert(sizeof(fx_dev) % 8 == 0, "descriptor copied as 8-byte words");
 
 // ---- TMA-staged persistent form -------------------------------------------
 // One block per SM slot loops over the domain's tiles. Thread 0 loads the
-// stencil of the block's next tile into the other of two shared-memory
-// stages with TMA (cp.async.bulk.tensor, completion counted on an mbarrier)
-// while the block computes the current one, so the halo reads of a tile
-// overlap the arithmetic of the previous tile.
+// tiles' stencils into two shared-memory stages with TMA (cp.async.bulk.tensor,
+// completion counted on an mbarrier), each as soon as its stage is free, two
+// tiles ahead, so the halo reads of a tile overlap the arithmetic of the ones
+// before it.
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
@@ -1942,7 +1942,7 @@ __global__ void __launch_bounds__(BX * BY, min_blocks<P32, BY>())
 // ---- TMA-staged persistent form for a batch --------------------------------
 // Each block walks a contiguous range of the packed tile table of all the
 // batch's domains (so it crosses few domain boundaries). Thread 0 stages the
-// stencil of the block's next tile with that domain's own tensor maps (a
+// stencil of the block's tile after next with that domain's own tensor maps (a
 // device array, one set per domain) while the block computes the current
 // tile; a domain without a solver step this launch (stopped, or no wet cell)
 // gets no stage. The domain's descriptor and step fields sit in shared
