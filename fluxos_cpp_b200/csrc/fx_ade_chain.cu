@@ -424,7 +424,8 @@ __device__ __forceinline__ Rec<T> make_rec(const fx_dev& d, const StepIn<T>& S, 
   const bool inflow_cell = gi == S.inflow_gi;
   const T hm = inflow_cell ? S.inflow_hm : w.h0;
   if (S.dilute) {
-    const bool use = interior & !(fl & FX_F_NODATA) & (w.hp != T(0));  // then hm >= hp > 0
+    // melt leaves hm >= hp > 0, evaporation may leave no depth: 0 / 0 then
+    const bool use = interior & !(fl & FX_F_NODATA) & (w.hp != T(0));
     // the melt depth the hydrodynamic step added (fx_hydro.cu melt32, melt_depth)
     T mi = w.mi;
     if constexpr (sizeof(T) == 8) {
@@ -438,7 +439,7 @@ __device__ __forceinline__ Rec<T> make_rec(const fx_dev& d, const StepIn<T>& S, 
       }
     }
     const T m = c * w.hp + (mi * S.mconc);
-    const bool some = use & (m != T(0));  // (an FP64 division of 0 takes the long way)
+    const bool some = use & ((m != T(0)) | !(hm > T(0)));  // (an FP64 division of 0 takes the long way)
     const T cd = tdiv(some ? m : T(1), some ? hm : T(1));
     c = some ? cd : (use ? m : c);
   }
