@@ -950,8 +950,11 @@ double fx_ade_active(int nr, int nc, int nchem, int steps) {
 // 63 steps), 2.1x at 1.6 (2048^2, 8), 1.28x at 3.2 (4096^2, 8), 1.17x at 3.5
 // (2048^2, 20), 1.04x at 5.1 (1500^2, 63), 0.75x at 6.1 (1024^2, 3 solutes,
 // 31); FP32 1.6x at 0.65, 1.4x at 1.6, 1.2x at 3.2, 1.13x at 6.1, 0.85x at 8
-// (2048^2, 63), 0.73x at 11 (4096^2, 31).
-bool fx_ade_use_chain(const fx_ade_caps& caps, double active) { return active <= caps.chain_active; }
+// (2048^2, 63), 0.73x at 11 (4096^2, 31). The results are the same bits, so the
+// option "ade_kernel" may take either.
+bool fx_ade_use_chain(const fx_ade_caps& caps, double active) {
+  return caps.kernel ? caps.kernel == 2 : active <= caps.chain_active;
+}
 
 void fx_launch_ade(const fx_dev* devs, const fx_unit* units, int nunits, const fx_ade_caps& caps, bool chain, bool prec32,
                    cudaStream_t s) {

@@ -836,6 +836,12 @@ int fx_set_option(fx_ctx* c, const char* name, long long v) {
     c->dev_version++;
     return FX_OK;
   }
+  if (!strcmp(name, "ade_kernel")) {
+    if (v < 0 || v > 2) return fx_fail(c, FX_ERR_ARG, "ade_kernel must be 0, 1 or 2");
+    c->ade_caps.kernel = (int)v;
+    c->graph_dirty = true;
+    return FX_OK;
+  }
   if (!strcmp(name, "tma")) {
     c->use_tma = v != 0;
     c->graph_dirty = true;

@@ -14,6 +14,7 @@
 struct fx_ade_caps {
   int sweep = 0, chain = 0;
   double chain_active = 0;  // the most units at work that the chain kernel takes (fx_ade_use_chain)
+  int kernel = 0;           // option "ade_kernel": 0 by the units at work, 1 the sweep kernel, 2 the chain kernel
 };
 
 struct fx_ctx {

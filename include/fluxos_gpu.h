@@ -144,7 +144,9 @@ int fx_set_melt_field(fx_ctx* ctx, const double* mult_grid);
  * 32 x tile_rows threads; by default the size of the grid decides); "tma" (1, the default: a persistent
  * hydrodynamic kernel whose blocks stage each tile's stencil into shared
  * memory by TMA while computing the previous tile; 0: one block per tile
- * loading its stencil itself). Results depend on neither.
+ * loading its stencil itself); "ade_kernel" (0, the default: the units at work
+ * decide which kernel sweeps the solutes; 1: the one with a warp per unit, 2:
+ * the one with a block per unit). Results depend on none of the three.
  * "fail_ade_waits" (1: for testing failure detection, the ADE sweep's
  * dependency waits are never satisfied, so they give up after a few
  * thousand polls, the kernels return, and the step returns FX_ERR_DEVICE
