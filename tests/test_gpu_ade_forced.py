@@ -116,6 +116,16 @@ def test_both_kernels_agree(nr, nc, dxy, nchem, in_flight, precision):
         assert np.isfinite(a[k]).all() and np.array_equal(a[k], b[k]), k
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_both_kernels_agree_on_a_large_grid(precision):
+    sc = S.fractal_scenario(1024, seed=3)
+    sc.d_coefs = [0.01, 0.05, 0.2]
+    S.wet_start(sc, depth=0.005)
+    a, b = _both(sc, precision, 31, 31)
+    for k in a:
+        assert np.array_equal(a[k], b[k]), k
+
+
 @pytest.mark.parametrize("kernel", KERNELS)
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_bounded_waits(precision, kernel):
