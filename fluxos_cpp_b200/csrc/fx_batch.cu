@@ -293,6 +293,9 @@ int fx_batch_set_option(fx_batch* b, const char* name, long long v) {
   } else if (!strcmp(name, "steps_in_flight")) {
     if (v < 1 || v > FX_MAX_SLOTS - 1) return fx_fail(nullptr, FX_ERR_ARG, "steps_in_flight must be 1..63");
     b->k_limit = (int)v;
+  } else if (!strcmp(name, "ade_kernel")) {
+    if (v < 0 || v > 2) return fx_fail(nullptr, FX_ERR_ARG, "ade_kernel must be 0, 1 or 2");
+    b->ade_caps.kernel = (int)v;
   } else if (!strcmp(name, "tma")) {
     b->use_tma = v != 0;
   } else {

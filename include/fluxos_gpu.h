@@ -204,7 +204,8 @@ int fx_batch_step(fx_batch* b, int nsteps, fx_status* st);
 void* fx_batch_stream(fx_batch* b);
 /* Options of the batch's launches: "tile_rows" (4, 8, 16, as for
  * fx_set_option), "steps_in_flight" (upper bound on the steps per graph,
- * 1..63; the members' own steps_in_flight bound it too) and "tma" (1, the
+ * 1..63; the members' own steps_in_flight bound it too), "ade_kernel" (as for
+ * fx_set_option, for the batch's sweep) and "tma" (1, the
  * default: the persistent TMA-staged hydrodynamic kernel when every member
  * allows it; 0: one block per tile; results are identical). */
 int fx_batch_set_option(fx_batch* b, const char* name, long long value);
