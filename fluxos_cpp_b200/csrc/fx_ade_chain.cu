@@ -784,11 +784,10 @@ __device__ __forceinline__ bool carry_warp(const fx_dev& d, const Unit<T>& U, Sm
       T cn = c.b + div_by(dc, c.h, c.y);
       cn = pmin(cmax, cn);
       cn = pmax(cn, cmin);
+      // (FP32 minima and maxima are the general form's, so cmax may be a NaN)
+      const T nan = sizeof(T) == 8 ? sum + have + cmax : sum + have;
       bool odd = c.fl & (K_DIV | K_KEEP);
-      if constexpr (sizeof(T) == 8) {  // (FP32 minima and maxima are the general form's)
-        const T nan = sum + have + cmax;
-        odd = odd | !(nan == nan) | div_far(dc) | (!pow2 & div_far(flux));
-      }
+      odd = odd | !(nan == nan) | div_far(dc) | (!pow2 & div_far(flux));
       if (__any_sync(0xffffffffu, odd)) {
         T gp = (c.fl & K_EAST) ? pfe0 : c.p1, gq = (c.fl & K_NORTH) ? qfn0 : c.p2;
         const T g = cell_general<T>(c.v0, W_pfe, o_qfn, c.l1, c.l2, dt, area, pow2 ? y_area : T(0), c.b, c.h,
