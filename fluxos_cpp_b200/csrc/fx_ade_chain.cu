@@ -461,7 +461,10 @@ __device__ __forceinline__ Rec<T> make_rec(const fx_dev& d, const StepIn<T>& S, 
     far = interior & wet2 & (div_far(ch) | !ok);
   }
   r.y = recip(r.hd);
-  b = wet2 ? div_by(ch, r.hd, r.y) : (dry ? T(0) : c);
+  T bw = div_by(ch, r.hd, r.y);
+  // a threshold of 0 leaves cells wet without water; their quotient is NaN
+  if constexpr (sizeof(T) == 4) bw = h != T(0) ? bw : __int_as_float(0x7fffffff);
+  b = wet2 ? bw : (dry ? T(0) : c);
   b = S.sweep ? b : c;
   T vol = (b * h) * S.area;
   v0 = div_by(vol, S.dt, S.y_dt);
