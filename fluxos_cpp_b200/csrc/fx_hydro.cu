@@ -811,6 +811,12 @@ __device__ __forceinline__ bool dd_le_hdry(const fx_dev& d, float eta, float lo)
   if (eta < d.f.hdry_lo) return true;
   return fx_dd_val(eta, lo) <= d.hdry;
 }
+// Above it: not the opposite of the one before, as neither holds for a NaN.
+__device__ __forceinline__ bool dd_gt_hdry(const fx_dev& d, float eta, float lo) {
+  if (eta > d.f.hdry_hi) return true;
+  if (eta < d.f.hdry_lo) return false;
+  return fx_dd_val(eta, lo) > d.hdry;
+}
 __device__ __forceinline__ bool dd_lt_hdry(const fx_dev& d, float eta, float lo) {
   if (eta > d.f.hdry_hi) return false;
   if (eta < d.f.hdry_lo) return true;
@@ -1358,7 +1364,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     d.qy_f[pcur + gi] = qy;
     const uint8_t fl1 = (fl & (FX_F_WALL | FX_F_NODATA)) | ((fl & FX_F_LDRY) ? FX_F_LDRY_PREV : 0) | ld;
     d.flags[scur + gi] = fl1;
-    if (computed && (d.store_all_fluxes || dd_le_hdry(d, eta, lo))) {
+    if (computed && (d.store_all_fluxes || !dd_gt_hdry(d, eta, lo))) {
       d.fe2_f[gi] = o[1];
       d.fe3_f[gi] = o[2];
       d.fn2_f[gi] = o[4];
@@ -1366,7 +1372,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     }
     // fe_1 and fn_1 of every cell go to this step's slot, kept ones too
     put_rec32(d, scur + gi, h0v, h, hpv, miv, o[0], o[3], fl1);
-    wet = eta > 0.0f && !dd_le_hdry(d, eta, lo);
+    wet = eta > 0.0f && dd_gt_hdry(d, eta, lo);
   }
   courant_tile32(d, wet, eta, lo, qx, qy, acc);
   acc.melt += bmelt;
