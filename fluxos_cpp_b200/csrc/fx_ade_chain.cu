@@ -477,7 +477,7 @@ __device__ __forceinline__ Rec<T> make_rec(const fx_dev& d, const StepIn<T>& S, 
     r.hd = h;
   }
   r.b = interior ? b : T(0);
-  r.v0 = interior ? v0 : T(0);
+  r.v0 = interior ? v0 : T(0) * h;  // of a ghost cell 0, or NaN with no number for its depth
   r.qx = w.fe;
   r.qy = w.fn;
   r.soil = T(0);
