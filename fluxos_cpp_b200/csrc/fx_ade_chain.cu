@@ -439,7 +439,8 @@ __device__ __forceinline__ Rec<T> make_rec(const fx_dev& d, const StepIn<T>& S, 
       }
     }
     const T m = c * w.hp + (mi * S.mconc);
-    const bool some = use & ((m != T(0)) | !(hm > T(0)));  // (an FP64 division of 0 takes the long way)
+    // an FP64 division of 0 takes the long way; in FP32 0 over a subnormal depth is NaN (trcp)
+    const bool some = use & ((sizeof(T) == 4) | (m != T(0)) | !(hm > T(0)));
     const T cd = tdiv(some ? m : T(1), some ? hm : T(1));
     c = some ? cd : (use ? m : c);
   }

@@ -48,3 +48,26 @@ def test_a_cell_that_loses_its_last_water(nr, nc, dxy, conc, precision, tmp_path
         want, got = (a[1:-1, 1:-1] for a in (ora.grid("conc"), d.download("conc")))
         assert np.array_equal(np.isnan(want), np.isnan(got)) and np.array_equal(np.isinf(want), np.isinf(got)), n
     d.close()
+
+
+@pytest.mark.parametrize("nr,nc,dxy", [(31, 40, 3), (62, 33, 2)])
+def test_subnormal_depths_in_fp32(nr, nc, dxy):
+    """The FP32 state's reciprocal of a subnormal depth is infinite, so a mass
+    of 0 diluted over one is NaN: from both kernels of the sweep."""
+    rng = np.random.default_rng(nr)
+    sc = _scenario(nr, nc, dxy, 1.0)
+    sc.meteo = ((0.0, 0.0, 0.0), (1e5, 0.0, 0.0))
+    sc.dem = np.full((nr, nc), 1e-50)  # a level of 1e-40 is a depth of 1e-40
+    sc.init_h = np.where(rng.random((nr, nc)) < 0.5, 1e-40, rng.uniform(0.001, 0.05, (nr, nc)))
+    sc.init_conc = [rng.uniform(0, 2, (nr, nc)) * (rng.random((nr, nc)) < 0.5)]
+    out = []
+    for kernel in (1, 2):
+        d = S.make_domain(sc, precision="fp32")
+        d.set_option("ade_kernel", kernel)
+        for n in (1, 4):
+            d.step(n)
+            out.append(d.download("conc"))
+        d.close()
+    assert np.isnan(out[0]).any()
+    for a, b in zip(out[:2], out[2:]):
+        assert np.array_equal(a, b, equal_nan=True)
