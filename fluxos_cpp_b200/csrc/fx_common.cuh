@@ -90,6 +90,7 @@ struct fx_ctl {
 struct fx_f32 {
   float hdry;              // dry threshold
   float hdry_lo, hdry_hi;  // outside of these an FP32 depth decides the threshold tests (fx_hydro.cu)
+  int below_zero;          // the threshold is: every cell is above it
   float ks, gaccl, nueml, dxy, inv_dxy, area;
 };
 
@@ -216,6 +217,7 @@ inline void fx_set_f32(fx_dev& d) {
   const double band = (d.hdry < 0 ? -d.hdry : d.hdry) * 0x1p-19;
   d.f.hdry_lo = (float)(d.hdry - band);
   d.f.hdry_hi = (float)(d.hdry + band);
+  d.f.below_zero = d.hdry < 0;
   d.f.ks = (float)d.ks;
   d.f.gaccl = (float)d.gaccl;
   d.f.nueml = (float)d.nueml;

@@ -1372,7 +1372,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
     }
     // fe_1 and fn_1 of every cell go to this step's slot, kept ones too
     put_rec32(d, scur + gi, h0v, h, hpv, miv, o[0], o[3], fl1);
-    wet = eta > 0.0f && dd_gt_hdry(d, eta, lo);
+    wet = d.f.below_zero || (eta > 0.0f && dd_gt_hdry(d, eta, lo));
   }
   courant_tile32(d, wet, eta, lo, qx, qy, acc);
   acc.melt += bmelt;
