@@ -721,7 +721,7 @@ __device__ __forceinline__ bool carry_warp(const fx_dev& d, const Unit<T>& U, Sm
   // its west cell for lane + 1
   T o_c = T(0), o_pfe = T(0), o_qfn = T(0);
   const T dt = U.S.dt, dxy = U.S.dxy, area = U.S.area, y_area = U.S.y_area;
-  const bool pow2 = U.S.pow2, wintra = U.S.wintra;
+  const bool pow2 = U.S.pow2, wintra = U.S.wintra, sweep = U.S.sweep;
   const long long ld = d.ld;
   for (int q = 0; q < U.rounds; ++q, ++k_round) {
     if (!wait_round<KR>(M, M.k_full, k_round)) return false;
@@ -793,10 +793,11 @@ __device__ __forceinline__ bool carry_warp(const fx_dev& d, const Unit<T>& U, Sm
       bool odd = c.fl & (K_DIV | K_KEEP);
       odd = odd | !(nan == nan) | div_far(dc) | (!pow2 & div_far(flux));
       if (__any_sync(0xffffffffu, odd)) {
-        T gp = (c.fl & K_EAST) ? pfe0 : c.p1, gq = (c.fl & K_NORTH) ? qfn0 : c.p2;
-        const T g = cell_general<T>(c.v0, W_pfe, o_qfn, c.l1, c.l2, dt, area, pow2 ? y_area : T(0), c.b, c.h,
-                                    fmax(wb1, c.cmax), fmin(wb2, c.cmin), gp, gq);
         const bool flow = (c.fl & (K_KEEP | K_DRY | K_VALID)) == K_VALID;
+        T g = T(0), gp = (c.fl & K_EAST) ? pfe0 : c.p1, gq = (c.fl & K_NORTH) ? qfn0 : c.p2;
+        if (sweep)  // a step without one keeps every cell (700 x 700, two solutes, FP64 1.06 ms; 2.67 with the call)
+          g = cell_general<T>(c.v0, W_pfe, o_qfn, c.l1, c.l2, dt, area, pow2 ? y_area : T(0), c.b, c.h,
+                              fmax(wb1, c.cmax), fmin(wb2, c.cmin), gp, gq);
         cn = flow ? g : ((c.fl & K_KEEP) ? c.b : T(0));
         pl = flow ? gp : T(0);
         ql = flow ? gq : T(0);
