@@ -104,9 +104,15 @@ static int rebuild(fx_batch* b) {
   // it waits for (fx_unit_order.h). Twelve domains of 257^2 to 1,600^2 cells in
   // FP32 take 1.55 ms a step, everything included, with a unit of each domain
   // in turn and these step by step, and 1.14 ms so.
-  std::stable_sort(units.begin(), units.end(), [&](const fx_unit& x, const fx_unit& y) {
-    return fx_ade_start(x.jj, x.s) - slack[x.dom] < fx_ade_start(y.jj, y.s) - slack[y.dom];
-  });
+  struct Timed {
+    double at;
+    fx_unit unit;
+  };
+  std::vector<Timed> order;
+  order.reserve(units.size());
+  for (const fx_unit& u : units) order.push_back(Timed{fx_ade_start(u.jj, u.s) - slack[u.dom], u});
+  std::stable_sort(order.begin(), order.end(), [](const Timed& x, const Timed& y) { return x.at < y.at; });
+  for (size_t i = 0; i < units.size(); ++i) units[i] = order[i].unit;
   int rc;
   if ((rc = grow(b, (void**)&b->d_devs, &b->cap_devs, sizeof(fx_dev) * std::max(n, 1)))) return rc;
   if ((rc = grow(b, (void**)&b->d_tiles, &b->cap_tiles, sizeof(fx_tile) * std::max<size_t>(tiles.size(), 1))))
@@ -143,10 +149,10 @@ static int rebuild(fx_batch* b) {
   FXB_CK(b, cudaStreamSynchronize(b->stream));
   b->ntiles = (int)tiles.size();
   b->nunits = (int)units.size();
-  if (fx_ade_caps_for(n > 0 && b->doms[0]->d.prec32 != 0, &b->ade_caps) != 0) {
-    int r = fx_fail(nullptr, FX_ERR_CUDA, "occupancy query for the ADE sweep failed");
-    b->err = fx_last_error(nullptr);
-    return r;
+  if (n) {  // the members' device and precision are the batch's
+    const int kernel = b->ade_caps.kernel;
+    b->ade_caps = b->doms[0]->ade_caps;
+    b->ade_caps.kernel = kernel;
   }
   double active = 0.0;
   for (fx_ctx* c : b->doms) active += c->p.ade ? fx_ade_active(c->g.nrows, c->g.ncols, c->g.nchem, b->K) : 0.0;
