@@ -53,8 +53,8 @@ constexpr int RING = 4;       // per-lane prefetch slots (a power of two); a dee
                               // memory from L1, which the lanes' skewed reads depend on (measured:
                               // 8 slots made the FP64 sweep 2.5x slower)
 // CHUNK: steps between progress checks and publications. A publication makes
-// the warp wait for its last writes; the lag between strips is
-// 2 * CHUNK + ROWS - 1 warp steps. DIST: prefetch distance in columns (< RING).
+// the warp wait for its last writes; a strip waits for a count of its west
+// strip that is 2 * CHUNK + ROWS - 1 warp steps ahead. DIST: prefetch distance in columns (< RING).
 // FP32 sweeps are many warps wide when they come here (fx_ade_use_chain) and
 // can do with the longer lag: ms a step with 4 and 2, 8 and 3, 16 and 3, at
 // 4096^2 cells, 63 steps 0.545, 0.484, 0.462; 2048^2, 63 steps 0.199, 0.186,
@@ -931,8 +931,15 @@ static size_t ade_smem(bool prec32) {
 }
 
 // Warp steps after the start of a launch until unit (jj, s) can start, when only
-// its dependencies hold it back: a strip follows its west strip by about 37, a
-// step the step before by about 48; and until the last unit ends.
+// its dependencies hold it back, and until the last unit ends: one model for
+// both kernels and precisions, in which a strip follows its west strip by 37
+// (2 * 4 + 29, the count a unit of the FP64 sweep waits for) and a step the
+// step before by 48. Launches on an otherwise empty GPU show 53 warp steps
+// between strips in FP64 (both kernels), 74 (sweep kernel) and 78 (chain
+// kernel) in FP32, as a count is known only some rounds after it is reached,
+// and 20 to 47 between steps of one strip. The model orders the units
+// (fx_unit_order.h, fx_batch.cu), where any weights of this kind are valid, and
+// scales fx_ade_active, whose lines below were measured with it.
 double fx_ade_start(int jj, int s) { return 48.0 * jj + 37.0 * s; }
 double fx_ade_span(int nr, int nc, int steps) {
   return fx_ade_start(steps, (nr + fxade::ROWS - 1) / fxade::ROWS) + nc;
@@ -943,15 +950,15 @@ double fx_ade_active(int nr, int nc, int nchem, int steps) {
   const double strips = (nr + fxade::ROWS - 1) / fxade::ROWS, tw = nc + fxade::ROWS - 1;
   return steps * nchem * strips * tw / fx_ade_span(nr, nc, steps);
 }
-// Which kernel. The chain kernel (a block per unit) takes a unit through its
-// warp steps 3 to 5 times faster but holds 2 (FP64) or 3 (FP32) units per SM
-// against 12, so it wins until the units at work are a few times its own. Its
-// gain over the sweep kernel at so many units per SM: FP64 2.3x at 0.65 (400^2,
-// 63 steps), 2.1x at 1.6 (2048^2, 8), 1.28x at 3.2 (4096^2, 8), 1.17x at 3.5
-// (2048^2, 20), 1.04x at 5.1 (1500^2, 63), 0.75x at 6.1 (1024^2, 3 solutes,
-// 31); FP32 1.6x at 0.65, 1.4x at 1.6, 1.2x at 3.2, 1.13x at 6.1, 0.85x at 8
-// (2048^2, 63), 0.73x at 11 (4096^2, 31). The results are the same bits, so the
-// option "ade_kernel" may take either.
+// Which kernel. The chain kernel (a block per unit) takes a unit alone through
+// its warp steps 2.7 (FP32) to 3.5 (FP64) times faster but holds 3 (FP32) or 2
+// units per SM against 12, so it wins until the units at work are a few times
+// its own. Its gain over the sweep kernel at so many units per SM: FP64 2.4x at
+// 0.65 (400^2, 63 steps), 2.2x at 1.6 (2048^2, 8), 1.6x at 3.2 (4096^2, 8), 1.5x
+// at 3.5 (2048^2, 20), 1.04x at 5.1 (1500^2, 63), 0.74x at 6.1 (1024^2, 3
+// solutes, 31); FP32 1.8x at 0.65, 1.4x at 1.6, 1.2x at 3.2 and at 5.1, 1.14x
+// at 6.1, 0.82x at 8 (2048^2, 63), 0.74x at 11 (4096^2, 31). The results are the
+// same bits, so the option "ade_kernel" may take either.
 bool fx_ade_use_chain(const fx_ade_caps& caps, double active) {
   return caps.kernel ? caps.kernel == 2 : active <= caps.chain_active;
 }

@@ -28,10 +28,12 @@
 //     during the launch) and boundary columns into shared rings; the publisher
 //     warp makes the carry warp's progress known. So no fence, poll or global
 //     load sits in the chain.
-// A strip alone takes 0.26 us (FP32) and 0.52 us (FP64) a warp step; one warp
-// that does all of it in turn (fx_ade.cu) takes 2.0 and 4.0 us. Of a carry
-// warp's 500 cycles (FP32) the dependent operations themselves are about 260
-// (measured alone on registers), the rest is votes, shared reads and waits.
+// A strip alone takes 0.27 us (FP32) and 0.53 us (FP64) a warp step, 540 and
+// 1,040 cycles; one warp that does all of it in turn (fx_ade.cu) 0.73 and 1.85
+// us. The cell's dependent operations alone, on registers, measure 260 and 430
+// cycles, with the two votes 290 and 500; the rest is shared reads and waits.
+// Eight steps of eight strips, each unit on an SM of its own, take 0.50 and
+// 0.64 us a warp step.
 //
 // Steps in flight: as in fx_ade.cu, step j+1 of a strip follows step j a few
 // rounds behind on the same and the next strip, and add_meteo's dilution
@@ -49,7 +51,6 @@
 
 #include <algorithm>
 #include <type_traits>
-#include <vector>
 
 #include "fx_common.cuh"
 #include "fx_internal.h"

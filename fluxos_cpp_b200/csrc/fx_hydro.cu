@@ -162,7 +162,6 @@ __device__ void solver_wet(const fx_dev& d, const SM& S, const BED& bed, int sr,
   const int ES = sidx(sr + 1, sc - 1), EN = sidx(sr + 1, sc + 1), WN = sidx(sr - 1, sc + 1);
   auto ksat = [&](int k) { return (S.cls[k] & C_INT) ? d.ks : 0.0; };
   auto hat = [&](int r, int q) { return max0(S.z[sidx(r, q)] - bed(r, q)); };
-  const double kspl = ksat(P);
   const double nueml = d.nueml, cvdefl = d.cvdefl;
   const unsigned dx = d.dxy_u, dy = d.dxy_u;
   bool lroe = true;
@@ -1130,8 +1129,7 @@ __device__ __forceinline__ bool hydro_tile32(const fx_dev& d, const StepCtl& c, 
                                              HydroSmem32<BY, STAGED>& S, TilePart& acc, const unsigned char* stg, int bad, F stage_free) {
   using L = StageLayout<true, BY>;
   const StageOff so = stage_off(tile.bx);
-  constexpr int TY = Tile<BY>::TY, NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX;
-  constexpr int NTHREADS = Tile<BY>::NTHREADS;
+  constexpr int TY = Tile<BY>::TY;
   const int lx = threadIdx.x, ly = threadIdx.y;
   const int tid = ly * BX + lx;
   const int irow0 = 1 + tile.bx * TX, icol0 = 1 + tile.by * TY;
@@ -1433,8 +1431,7 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
   using SM = HydroSmem64<BY, STAGED>;
   using L = StageLayout<false, BY>;
   const StageOff so = stage_off(tile.bx);
-  constexpr int TY = Tile<BY>::TY, NSTEN = Tile<BY>::NSTEN, NFLUX = Tile<BY>::NFLUX;
-  constexpr int NTHREADS = Tile<BY>::NTHREADS;
+  constexpr int TY = Tile<BY>::TY;
   const int lx = threadIdx.x, ly = threadIdx.y;
   const int tid = ly * BX + lx;
   const int irow0 = 1 + tile.bx * TX, icol0 = 1 + tile.by * TY;
@@ -1716,8 +1713,7 @@ __device__ __forceinline__ bool hydro_tile64(const fx_dev& d, const StepCtl& c, 
 __device__ __forceinline__ void let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void follow() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// Reads the step's fields of the control block (written by k_finalize) into
-// shared memory, then runs the tile in the domain's precision.
+// One tile of a step without solver, in the domain's precision.
 template <bool P32, int BY>
 __device__ __forceinline__ void idle_tile(const fx_dev& d, const StepCtl& c, const fx_tile& tile, TilePart& acc) {
   if constexpr (P32) idle_tile32<BY>(d, c, tile, acc);
@@ -1734,6 +1730,8 @@ __device__ __forceinline__ bool hydro_tile(const fx_dev& d, const StepCtl& c, co
   else return hydro_tile64<BY, STAGED>(d, c, tile, S, acc, stg, bad, stage_free);
 }
 
+// Reads the step's fields of the control block (written by k_finalize) into
+// shared memory, then runs the tile.
 template <bool P32, int BY>
 __device__ __forceinline__ void hydro_block(const fx_dev& d, const fx_tile& tile, HydroSmem<P32, BY, false>& S,
                                             StepCtl& sc) {

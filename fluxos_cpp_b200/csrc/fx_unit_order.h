@@ -2,14 +2,14 @@
 // s of step jj; fx_ade.cu, fx_ade_chain.cu). Plain C++, for the kernels and
 // the host.
 //
-// A unit can start when its west strip of the same step is about 37 warp
-// steps along and its own strip of the step before about 48 (fx_ade_active),
-// so unit (jj, s) at about 48 jj + 37 s warp steps. Handed out step by step,
+// A unit can start when its west strip of the same step and its own strip of
+// the step before are some way along: in the model of fx_ade_start by 37 and 48
+// warp steps, so unit (jj, s) at 48 jj + 37 s. Handed out step by step,
 // the last strips of a step hold their warps or blocks for thousands of warp
 // steps before they can start, while units of later steps that could run are
 // not handed out yet (sweep of 4096 x 4096 cells, 20 steps in FP64 1.99 ms a
 // step, 63 in FP32 0.65; of 1000 x 700, 24 in FP64 0.190; in the order below
-// 1.50, 0.545 and 0.141). So units go out by t = jj + floor(3 s / 4), their start
+// 1.50, 0.545 and 0.141, all else equal). So units go out by t = jj + floor(3 s / 4), their start
 // in units of 48 warp steps, and within a t by step, then strip. Every unit
 // that one waits for, (jj, s - 1), (jj - 1, s) and (jj - 1, s + 1), comes
 // earlier: t is one less, or the same with a smaller step or strip.
